@@ -6,8 +6,10 @@
 // (lights.h:34-37) and the per-row sinf of the environment distribution (lights.h:70,94), plus the
 // luminance of each environment texel (math.h:112), so the device never needs those transcendentals.
 #include "device_scene.h"
+#include "tree_check.h"
 #include "wide_bvh.h"
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -125,6 +127,15 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
         } else {
             nodes4_.release();
         }
+        // Levels of the tree (children follow their parents).
+        std::vector<uint8_t> level(size_t(d.num_nodes), 1);
+        tree_depth_ = 1;
+        for (int32_t i = 0; i < d.num_nodes; i++) {
+            const uint8_t next = uint8_t(std::min<int>(level[size_t(i)] + 1, 255));
+            tree_depth_ = std::max<int>(tree_depth_, level[size_t(i)]);
+            if (d.nodes[i].lcount <= 0 && d.nodes[i].left >= 0) level[size_t(d.nodes[i].left)] = next;
+            if (d.nodes[i].rcount <= 0 && d.nodes[i].right >= 0) level[size_t(d.nodes[i].right)] = next;
+        }
         num_vertices_ = d.num_vertices;
         if (d.normals) {
             std::vector<float4> n(size_t(d.num_vertices));
@@ -233,7 +244,8 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.p_emissive = d.p_emissive;
     v.p_punctual = d.p_punctual;
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
-    v.bvh_depth = 0;
+    v.bvh_depth = tree_depth_;
+    v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_depth_, s) ? 1 : 0;
     {
         float lo[3] = {d.bounds_min.x, d.bounds_min.y, d.bounds_min.z}, hi[3] = {d.bounds_max.x, d.bounds_max.y, d.bounds_max.z};
         float inv[3];

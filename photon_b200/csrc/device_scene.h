@@ -103,6 +103,7 @@ private:
     float extent_ = 1.0f;
     int32_t num_vertices_ = 0;
     int32_t num_materials_ = 0;
+    int tree_depth_ = 0;
     void upload_shade_keys(const pt_material* materials, int32_t n, cudaStream_t s);
     float bounds_[6] = {0, 0, 0, 0, 0, 0};  // the scene box (lo xyz, hi xyz), for the light-group weights
 };

@@ -22,24 +22,60 @@ PT_HD int wrap_coord(int i, int n, bool repeat) {
     }
     return i < 0 ? 0 : (i >= n ? n - 1 : i);
 }
-PT_HD V4 sample_texture(const DevScene& s, int tex, V2 uv) {
-    int4 t = __ldg(s.textures + tex);
-    float x = uv.x * float(t.x) - 0.5f, y = uv.y * float(t.y) - 0.5f;
-    float fx = floorf(x), fy = floorf(y);
-    if (!(fabsf(fx) < 1e8f) || !(fabsf(fy) < 1e8f)) return {0, 0, 0, 1};
-    int x0 = int(fx), y0 = int(fy);
-    float tx = x - fx, ty = y - fy;
-    bool rep = (t.w & 1) != 0, srgb = (t.w & 2) != 0;
-    int xa = wrap_coord(x0, t.x, rep), xb = wrap_coord(x0 + 1, t.x, rep);
-    int ya = wrap_coord(y0, t.y, rep), yb = wrap_coord(y0 + 1, t.y, rep);
+// The wrapped coordinates of texels i and i + 1. A repeated power of two (the common size) wraps by a
+// mask; another one by one division, since the second coordinate follows from the first.
+PT_HD void wrap_pair(int i, int n, bool repeat, int& a, int& b) {
+    if (!repeat) {
+        a = wrap_coord(i, n, false);
+        b = wrap_coord(i + 1, n, false);
+        return;
+    }
+    a = (n & (n - 1)) == 0 ? i & (n - 1) : wrap_coord(i, n, true);
+    b = a + 1 == n ? 0 : a + 1;
+}
+// The four texels of a bilinear lookup and their weights; false where the coordinates are out of range.
+struct TexelQuad {
+    const uint32_t *a, *b, *c, *d;  // (xa, ya), (xb, ya), (xa, yb), (xb, yb)
+    float tx, ty;
+};
+PT_HD bool texel_quad(const DevScene& s, int4 t, V2 uv, TexelQuad& q) {
+    const float x = uv.x * float(t.x) - 0.5f, y = uv.y * float(t.y) - 0.5f;
+    const float fx = floorf(x), fy = floorf(y);
+    if (!(fabsf(fx) < 1e8f) || !(fabsf(fy) < 1e8f)) return false;
+    q.tx = x - fx;
+    q.ty = y - fy;
+    const bool rep = (t.w & 1) != 0;
+    int xa, xb, ya, yb;
+    wrap_pair(int(fx), t.x, rep, xa, xb);
+    wrap_pair(int(fy), t.y, rep, ya, yb);
     const uint32_t* base = s.texels + uint32_t(t.z);
-    V4 a = unpack_texel(__ldg(base + ya * t.x + xa), srgb, s.srgb_lut);
-    V4 b = unpack_texel(__ldg(base + ya * t.x + xb), srgb, s.srgb_lut);
-    V4 c = unpack_texel(__ldg(base + yb * t.x + xa), srgb, s.srgb_lut);
-    V4 d = unpack_texel(__ldg(base + yb * t.x + xb), srgb, s.srgb_lut);
-    V4 top = a * (1 - tx) + b * tx;
-    V4 bottom = c * (1 - tx) + d * tx;
-    return top * (1 - ty) + bottom * ty;
+    q.a = base + ya * t.x + xa;
+    q.b = base + ya * t.x + xb;
+    q.c = base + yb * t.x + xa;
+    q.d = base + yb * t.x + xb;
+    return true;
+}
+PT_HD V4 sample_texture(const DevScene& s, int tex, V2 uv) {
+    const int4 t = __ldg(s.textures + tex);
+    TexelQuad q;
+    if (!texel_quad(s, t, uv, q)) return {0, 0, 0, 1};
+    const bool srgb = (t.w & 2) != 0;
+    V4 a = unpack_texel(__ldg(q.a), srgb, s.srgb_lut);
+    V4 b = unpack_texel(__ldg(q.b), srgb, s.srgb_lut);
+    V4 c = unpack_texel(__ldg(q.c), srgb, s.srgb_lut);
+    V4 d = unpack_texel(__ldg(q.d), srgb, s.srgb_lut);
+    V4 top = a * (1 - q.tx) + b * q.tx;
+    V4 bottom = c * (1 - q.tx) + d * q.tx;
+    return top * (1 - q.ty) + bottom * q.ty;
+}
+// sample_texture(..).w alone, by the same operations.
+PT_HD float sample_alpha(const DevScene& s, int tex, V2 uv) {
+    TexelQuad q;
+    if (!texel_quad(s, __ldg(s.textures + tex), uv, q)) return 1.0f;
+    const float k = 1.0f / 255.0f;
+    const float a = float(__ldg(q.a) >> 24) * k, b = float(__ldg(q.b) >> 24) * k, c = float(__ldg(q.c) >> 24) * k, d = float(__ldg(q.d) >> 24) * k;
+    const float top = a * (1 - q.tx) + b * q.tx, bottom = c * (1 - q.tx) + d * q.tx;
+    return top * (1 - q.ty) + bottom * q.ty;
 }
 
 PT_HD V2 load_uv(const DevScene& s, int v) {
@@ -62,7 +98,7 @@ PT_HD bool alpha_passes(const DevScene& s, const float4* g, int material, float 
     if (base_tex >= 0 && s.uvs) {
         const float4 g3 = __ldg(g + 3);
         V2 uv = interp_uv(s, make_int4(__float_as_int(g3.x), __float_as_int(g3.y), __float_as_int(g3.z), 0), u, v);
-        alpha *= sample_texture(s, base_tex, uv).w;
+        alpha *= sample_alpha(s, base_tex, uv);
     }
     return alpha < m3.x;
 }

@@ -174,6 +174,9 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
         p.single_nodes = single_host->nodes;
         p.single_nodes4 = single_host->nodes4;
         p.single_tris = single_host->tris;
+        p.order_free = single_host->order_free;
+    } else {
+        p.order_free = order_free_ ? 1 : 0;
     }
     p.pb = pb_;
     p.ctr = ctr_.ptr;
@@ -921,7 +924,7 @@ void Renderer::trace_primary(const pt_camera& cam, int w, int h, uint32_t frame,
     const Tuning& t = engine_->tuning();
     const uint32_t pairs = t.packed ? uint32_t(std::clamp(t.pair_walk, 0, 64)) : 0u;  // the render's closest-hit walk
     PTW_CUDA(wf_trace_primary(scene_.device_view(), reinterpret_cast<const float*>(&cam), w, h, frame, seed, out.ptr, probe_claim_.ptr, pairs,
-                              stream_));
+                              scene_.view().order_free != 0, stream_));
     PTW_CUDA(cudaMemcpyAsync(hits4, out.ptr, out.bytes(), cudaMemcpyDeviceToHost, stream_));
     PTW_CUDA(cudaStreamSynchronize(stream_));
 }

@@ -101,6 +101,12 @@ public:
     // stay as they were set before begin().
     void update_scheduling(const Tuning& t);
 
+    // Whether every scene that multi-scene launches may meet is DevScene::order_free.
+    void set_order_free(bool all) {
+        order_free_ = all;
+        cont_params_.order_free = all ? 1 : 0;
+    }
+
     const Counters& last() const { return last_; }
 
     // Profiling (pt_set_profiling): per-kernel device time recorded by events inside the graphs,
@@ -139,6 +145,7 @@ private:
     cudaEvent_t ev_ = nullptr;
     // continuous mode
     WfParams cont_params_{};
+    bool order_free_ = false;
     int profile_flags_ = 0;
     std::vector<cudaEvent_t> prof_ev_;
     uint32_t tail_limit_ = 0;

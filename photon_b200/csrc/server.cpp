@@ -551,6 +551,7 @@ void Server::session_loop() {
                                      session_stream_));
             PTW_CUDA(cudaMemcpyAsync(session_views_.ptr, views.data(), views.size() * sizeof(DevView), cudaMemcpyHostToDevice,
                                      session_stream_));
+            session_engine_->set_order_free(std::all_of(table.begin(), table.end(), [](const DevScene& t) { return t.order_free != 0; }));
             session_engine_->run(session_scenes_.ptr, single, single >= 0 ? &table[size_t(single)] : nullptr, session_views_.ptr,
                                  int(views.size()), work);
             for (size_t k = 0; k < frames.size(); k++) {
@@ -671,6 +672,7 @@ void Server::upload_scene_table() {
     std::vector<DevScene> table;
     for (const auto& s : scenes_) table.push_back(s->view());
     PTW_CUDA(cudaMemcpyAsync(d_scenes_.ptr, table.data(), table.size() * sizeof(DevScene), cudaMemcpyHostToDevice, stream_));
+    engine_->set_order_free(std::all_of(table.begin(), table.end(), [](const DevScene& s) { return s.order_free != 0; }));
     scenes_dirty_ = false;
 }
 

@@ -456,6 +456,260 @@ __device__ __forceinline__ void walk_queue_pairs4(uint32_t n, uint32_t* claim, u
     }
 }
 
+// ---- the list walk -----------------------------------------------------------------------------------
+// The default walk of scenes whose tree may be walked out of order (DevScene::order_free). Photon's walk,
+// and the pair walk with it, holds a ray at a node until its leaf children are tested, because they may
+// lower tmax; but which hit a ray ends on depends on that only in rare cases that can be told, so here a
+// lane that meets leaf children puts them on its warp's list and walks on at once, and the warp tests the
+// listed triangles 32 at a time: every lane that has a ray visits nodes in every round, and a test round
+// has 32 (ray, triangle) pairs. The nodes a lane visits before its limit comes down cost about 4% more
+// visits.
+//
+// Why an answer is Photon's. The boxes are the BVH2's, nested (checked at upload, tree_check.cu), tested
+// by Photon's arithmetic, which is monotone in the bounds: a box that passes at some tmax has ancestors
+// that pass.
+//   Any hit: tmax never changes, so Photon tests the triangles of the same leaves, in another order.
+//   Closest hit: let T be the triangle of least distance t among those whose leaf box the ray enters.
+//   Photon's tmax is never below t before it tests T, so T is reached and the walk ends on it - unless
+//   another triangle with a distance between t and T's box entry (which rounding can put a little beyond
+//   t), or exactly t, was accepted first. This walk visits nodes in Photon's order and prunes later than
+//   Photon does, at (1 + 2^-10) of the least distance so far, so it tests every triangle that Photon tests
+//   and every such other one. If the second least distance it accepted is within 1 + 2^-14 of the least,
+//   or it accepted a triangle clearly ahead of its own box (one seen edge-on, whose distance is rounding),
+//   the ray is walked again in Photon's order: about one ray in 10,000.
+constexpr uint32_t kListCap = 128;  // entries of a warp's ring; a round of visits appends up to 64
+constexpr int kListStack = 12;      // stack entries per thread kept in shared memory (16: trace +0.5%)
+constexpr uint32_t kListVisits = 2; // rounds per step, per node visit of a pair walk's step (see walk_queue_list)
+constexpr float kPrune = 1.0f + 1.0f / 1024.0f;
+constexpr float kNearTie = 1.0f + 1.0f / 16384.0f;
+
+template <bool AnyHit, bool Single>
+struct ListSlots {
+    float4 o[32];                              // the lane's ray: origin
+    float4 d[32];                              // direction, limit on the distance
+    unsigned long long best[AnyHit ? 1 : 32];  // least accepted distance: its bits << 32 | triangle; ~0 none
+    const DevScene* scene[Single ? 1 : 32];
+    float2 uv[AnyHit ? 1 : 32];                // barycentrics of `best`
+    uint2 list[kListCap];                      // a leaf: (2 * node + side) << 5 | owner's lane, its box entry
+    uint8_t start[32];                         // a test round's leaves by their first pair
+    uint32_t mark[32];                         // any-hit: 1 once answered; closest: second least distance's bits
+};
+
+// Photon's walk of one ray, by one thread.
+__device__ __forceinline__ float4 exact_closest(const DevScene* s, V3 o, V3 d) {
+    int stack[kSmemStack];
+    TraversalCounters tc{0, 0, 0};
+    Hit h{kInf, -1, 0.0f, 0.0f};
+    traverse<false, false>(*s, o, d, kInf, h, stack, 1, &tc);
+    return make_float4(h.t, __int_as_float(h.tri), h.u, h.v);
+}
+
+// The finished closest-hit ray's (distance, triangle bits, u, v).
+template <bool Single>
+__device__ __forceinline__ float4 list_hit(const ListSlots<false, Single>& ls, uint32_t lane, const DevScene* scene) {
+    const unsigned long long key = ls.best[lane];
+    if (key == ~0ull) return make_float4(kInf, __int_as_float(-1), 0.0f, 0.0f);
+    const float t = __uint_as_float(uint32_t(key >> 32));
+    if (__uint_as_float(ls.mark[lane]) <= t * kNearTie) return exact_closest(scene, xyz(ls.o[lane]), xyz(ls.d[lane]));
+    const float2 uv = ls.uv[lane];
+    return make_float4(t, __int_as_float(int(uint32_t(key))), uv.x, uv.y);
+}
+
+// Tests triangle i for the ray of lane k (`on`: this lane has a pair); `entry`: its leaf box's.
+template <bool AnyHit, bool Single>
+__device__ __forceinline__ void list_test(ListSlots<AnyHit, Single>& ls, bool on, uint32_t k, int i, float entry, const WalkScene& uniform) {
+    bool accepted = false;
+    unsigned long long key = ~0ull;
+    float t, tu, tv;
+    if (on) {
+        const float4 o = ls.o[k], d = ls.d[k];
+        const DevScene* sc = Single ? uniform.scene : ls.scene[k];
+        const float4* g = (Single ? uniform.tris : sc->tris) + kTriStride * i;
+        float4 g0, g1;
+        ldg_pair(g, g0, g1);
+        const float4 g2 = __ldg(g + 2);
+        accepted = tri_intersect(g0, g1, g2, xyz(o), xyz(d), d.w, t, tu, tv) &&
+                   !((__float_as_int(g1.w) & 1) && alpha_passes(*sc, g, __float_as_int(g0.w), tu, tv));
+        if (accepted) {
+            if (AnyHit) {
+                ls.mark[k] = 1u;
+            } else {
+                key = (unsigned long long)__float_as_uint(t) << 32 | uint32_t(i);
+                const unsigned long long old = atomicMin(&ls.best[k], key);
+                const unsigned long long other = old > key ? old : key;
+                if (t < entry * (1.0f - 1.0f / 16384.0f)) atomicMin(&ls.mark[k], 0u);
+                else if (other != ~0ull) atomicMin(&ls.mark[k], uint32_t(other >> 32));
+            }
+        }
+    }
+    __syncwarp();
+    if (!AnyHit) {
+        if (accepted && ls.best[k] == key) ls.uv[k] = make_float2(tu, tv);
+        __syncwarp();
+    }
+}
+
+// Tests m listed leaves (at most 32, one per lane) from list position `head` on, 32 pairs at a time; a
+// leaf entered beyond its owner's present limit is dropped.
+template <bool AnyHit, bool Single>
+__device__ __forceinline__ void list_leaves(ListSlots<AnyHit, Single>& ls, uint32_t head, uint32_t m, const WalkScene& uniform) {
+    const uint32_t lane = lane_id(), upto = 0xffffffffu >> (31u - lane);
+    uint32_t count = 0, owner = 0;
+    int first = 0;
+    float entry = 0.0f;
+    if (lane < m) {
+        const uint2 e = ls.list[(head + lane) & (kListCap - 1)];
+        owner = e.x & 31u;
+        entry = __uint_as_float(e.y);
+        if (entry <= ls.d[owner].w) {
+            const float4* np = (Single ? uniform.nodes : ls.scene[owner]->nodes) + 2 * size_t(e.x >> 5);
+            first = __float_as_int(__ldg(np).w);
+            count = uint32_t(__float_as_int(__ldg(np + 1).w));
+        }
+    }
+    uint32_t incl = count;
+#pragma unroll
+    for (uint32_t s = 1; s < 32; s <<= 1) {
+        const uint32_t x = __shfl_up_sync(kFull, incl, s);
+        if (lane >= s) incl += x;
+    }
+    const uint32_t excl = incl - count, total = __shfl_sync(kFull, incl, 31);
+    for (uint32_t base = 0; base < total; base += 32) {
+        // The leaf of pair base + lane: the last one with triangles that starts up to there, in this round
+        // (its start bit in `starts`, its lane in ls.start) or before it.
+        const bool here = count && excl - base < 32u;
+        const uint32_t starts = __reduce_or_sync(kFull, here ? 1u << (excl - base) : 0u) & upto;
+        const uint32_t before = __ballot_sync(kFull, count && excl < base);
+        if (here) ls.start[excl - base] = uint8_t(lane);
+        __syncwarp();
+        const uint32_t j = starts ? uint32_t(ls.start[31 - __clz(int(starts))]) : uint32_t(31 - __clz(int(before))) & 31u;
+        const int off = __shfl_sync(kFull, first - int(excl), int(j));
+        const uint32_t k = __shfl_sync(kFull, owner, int(j));
+        const float e = AnyHit ? 0.0f : __shfl_sync(kFull, entry, int(j));
+        list_test<AnyHit, Single>(ls, base + lane < total, k, off + int(base + lane), e, uniform);
+    }
+}
+
+// Persistent walk over a ray queue in warp steps: up to kListVisits x `visits` rounds in which every lane
+// with a node visits it, then the listed leaves, 32 at a time (fewer stay listed, unless fewer than
+// `refill` lanes have a node to visit: the others wait for their leaves). Refill as in walk_queue. A lane
+// does not wait for its leaves, so a step is best longer than a pair walk's: per 1080p frame of the 262K
+// scene the trace took 21.9, 21.6, 21.5 and 21.3 ms with 6, 8, 10 and 13 rounds.
+// begin(i, o, d, tmax, nodes, scene) loads queue entry i and returns its record; end(record, slots, lane)
+// consumes the finished ray.
+template <bool AnyHit, bool Single, typename Begin, typename End>
+__device__ __forceinline__ void walk_queue_list(uint32_t n, uint32_t* claim, uint32_t refill, uint32_t visits, int* stack, int stride,
+                                                ListSlots<AnyHit, Single>& ls, const WalkScene& uniform, Begin begin, End end) {
+    int overflow[kStackSize - kListStack];
+    RaySlab rs{};
+    float limit = 0.0f;
+    const float4* nodes = uniform.nodes;
+    int node = -1, sp = 0;
+    uint32_t idx = 0, head = 0, tail = 0, last = 0;  // list positions count on; modulo kListCap in the ring
+    bool live = false, drained = false;
+    const uint32_t lane = lane_id(), below = (1u << lane) - 1u;
+    for (;;) {
+        uint32_t act = __ballot_sync(kFull, live);
+        if (!drained && uint32_t(__popc(act)) < refill) {
+            const uint32_t idle = ~act, want = uint32_t(__popc(idle));
+            uint32_t base = 0;
+            if (lane == 0) base = atomicAdd(claim, want);
+            base = __shfl_sync(kFull, base, 0);
+            drained = base + want >= n;
+            if (!live) {
+                const uint32_t r = base + uint32_t(__popc(idle & below));
+                if (r < n) {
+                    V3 o, d;
+                    const DevScene* scene = nullptr;
+                    idx = begin(r, o, d, limit, nodes, scene);
+                    rs = ray_slab(o, V3{safe_inv(d.x), safe_inv(d.y), safe_inv(d.z)});
+                    ls.o[lane] = make_float4(o.x, o.y, o.z, 0.0f);
+                    ls.d[lane] = make_float4(d.x, d.y, d.z, limit);
+                    ls.mark[lane] = AnyHit ? 0u : ~0u;
+                    if (!AnyHit) ls.best[lane] = ~0ull;
+                    if (!Single) ls.scene[lane] = scene;
+                    stack[0] = -1;  // the bottom: popped once nothing is left
+                    node = 0;
+                    sp = 1;
+                    last = head;
+                    live = true;
+                }
+            }
+            act = __ballot_sync(kFull, live);
+        }
+        if (act == 0) break;
+        for (uint32_t it = 0; it < kListVisits * visits && tail - head <= kListCap - 64; it++) {
+            bool leaf0 = false, leaf1 = false;
+            float t0 = 0.0f, t1 = 0.0f;
+            uint32_t at = 0;
+            if (node >= 0) {
+                const float4* np = (Single ? uniform.nodes : nodes) + 4 * size_t(node);
+                float4 n0, n1, n2, n3;
+                ldg_pair(np, n0, n1);
+                ldg_pair(np + 2, n2, n3);
+                t0 = box_entry3(n0, n1, rs, limit);
+                t1 = box_entry3(n2, n3, rs, limit);
+                const int c0 = __float_as_int(n1.w), i0 = __float_as_int(n0.w), c1 = __float_as_int(n3.w), i1 = __float_as_int(n2.w);
+                const bool h0 = t0 != kInf, h1 = t1 != kInf;
+                at = uint32_t(node) << 6 | lane;
+                leaf0 = h0 && c0 > 0;
+                leaf1 = h1 && c1 > 0;
+                const bool in0 = h0 && c0 <= 0 && i0 >= 0 && t0 < limit, in1 = h1 && c1 <= 0 && i1 >= 0 && t1 < limit;
+                if (in0 || in1) {
+                    const bool second = in1 && (!in0 || t0 > t1);  // side 1 next
+                    if (in0 && in1) {
+                        const int far = second ? i0 : i1;
+                        if (sp < kListStack) stack[sp * stride] = far;
+                        else overflow[sp - kListStack] = far;
+                        sp++;
+                    }
+                    node = second ? i1 : i0;
+                } else {
+                    --sp;
+                    node = sp < kListStack ? stack[sp * stride] : overflow[sp - kListStack];
+                }
+            }
+            const uint32_t l0 = __ballot_sync(kFull, leaf0), l1 = __ballot_sync(kFull, leaf1);
+            if (l0 | l1) {
+                const uint32_t p0 = tail + uint32_t(__popc(l0 & below)), n0 = uint32_t(__popc(l0)), p1 = tail + n0 + uint32_t(__popc(l1 & below));
+                if (leaf0) {
+                    ls.list[p0 & (kListCap - 1)] = make_uint2(at, __float_as_uint(t0));
+                    last = p0 + 1;
+                }
+                if (leaf1) {
+                    ls.list[p1 & (kListCap - 1)] = make_uint2(at | 32u, __float_as_uint(t1));
+                    last = p1 + 1;
+                }
+                tail += n0 + uint32_t(__popc(l1));
+            }
+        }
+        __syncwarp();
+        const bool flush = uint32_t(__popc(__ballot_sync(kFull, node >= 0))) < refill;
+        while (tail - head >= 32u || (flush && tail != head)) {
+            const uint32_t m = min(tail - head, 32u);
+            list_leaves<AnyHit, Single>(ls, head, m, uniform);
+            head += m;
+        }
+        if (live) {
+            if (AnyHit) {
+                if (ls.mark[lane]) {
+                    node = -1;
+                    ls.d[lane].w = -1.0f;  // its leaves still listed are dropped
+                }
+            } else {
+                const float t = __uint_as_float(uint32_t(ls.best[lane] >> 32));  // (a NaN without a hit)
+                limit = t < kInf ? fminf(t * kPrune, kInf) : limit;
+                ls.d[lane].w = limit;
+            }
+            if (node < 0 && int(head - last) >= 0) {
+                end(idx, ls, lane);
+                live = false;
+            }
+        }
+        __syncwarp();
+    }
+}
+
 // The scene arrays of a launch whose views all use one scene (the renderer), or null arrays (the
 // server: each ray's scene comes from its view).
 __device__ __forceinline__ WalkScene single_walk_scene(const WfParams& P, bool wide) {
@@ -544,6 +798,38 @@ __global__ void __maxnreg__(56) k_trace_pairs(const __grid_constant__ WfParams P
         warp_add_u64(&c->trace_lane_steps, tc.steps);
         if (lane_id() == 0) atomicAdd(&c->trace_warp_steps, (unsigned long long)warp_steps);
     }
+}
+
+// The closest-hit list walk (walk_queue_list): the same hits as k_trace and k_trace_pairs. Dynamic shared
+// memory: the stacks, then one ListSlots per warp. Bound by issue and by the L1's wavefronts together (73%
+// and 66% of their peaks on camera rays, 22 of 32 lanes per instruction against the pair walk's 18). 64
+// registers: the rare exact walk inlined at a ray's end spills in the round at 56 (trace 22.5 ms), and 72
+// cost a block per SM (21.8). Per 1080p frame of the 262K scene: 23.5 (pair walk) -> 21.4 ms; 1.05M
+// triangles, 1280x720 at 8 spp: 7.8 -> 7.2 ms.
+template <bool Single>
+__global__ void __maxnreg__(64) k_trace_list(const __grid_constant__ WfParams P) {
+    extern __shared__ int list_smem[];
+    using S = ListSlots<false, Single>;
+    S& ls = reinterpret_cast<S*>(list_smem + kListStack * blockDim.x)[threadIdx.x >> 5];
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t p = c->parity, n = c->count[p];
+    const WalkScene uni = single_walk_scene(P, false);
+    walk_queue_list<false, Single>(
+        n, &c->fetch[1], P.trace_refill, P.pair_visits, list_smem + threadIdx.x, blockDim.x, ls, uni,
+        [&](uint32_t i, V3& o, V3& d, float& tmax, const float4*& nodes, const DevScene*& scene) {
+            if (!Single) {
+                scene = &P.scenes[P.views[P.pb.id[p][i].x].scene];
+                nodes = scene->nodes;
+            }
+            o = xyz(P.pb.o[p][i]);
+            d = xyz(P.pb.d[p][i]);
+            tmax = kInf;
+            return i;
+        },
+        [&](uint32_t i, const S& sl, uint32_t lane) {
+            P.pb.hit[i] = list_hit(sl, lane, Single ? uni.scene : sl.scene[lane]);
+        });
 }
 
 // Sort key of a continuing ray: direction octant, then the Morton code of its origin's cell in the
@@ -1052,6 +1338,36 @@ __global__ void __maxnreg__(56) k_shadow_pairs(const __grid_constant__ WfParams 
     }
 }
 
+// The any-hit list walk: the same answers as k_shadow and k_shadow_pairs. Per 1080p frame of the 262K
+// scene: 10.9 (pair walk) -> 9.4 ms. (Visiting the farther child first, which any-hit answers allow: 9.9.)
+template <bool Single>
+__global__ void __maxnreg__(56) k_shadow_list(const __grid_constant__ WfParams P) {
+    extern __shared__ int list_smem[];
+    using S = ListSlots<true, Single>;
+    S& ls = reinterpret_cast<S*>(list_smem + kListStack * blockDim.x)[threadIdx.x >> 5];
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t n = c->shadow_count;
+    const ShadowQueue sq{P, c->parity ^ 1u, c->shadow_sorting != 0};
+    walk_queue_list<true, Single>(
+        n, &c->fetch[3], P.shadow_refill, P.pair_visits, list_smem + threadIdx.x, blockDim.x, ls, single_walk_scene(P, false),
+        [&](uint32_t i, V3& o, V3& d, float& tmax, const float4*& nodes, const DevScene*& scene) {
+            const uint32_t j = sq.record(i);
+            const float4 a = P.pb.sh0[j];
+            o = xyz(a);
+            d = xyz(P.pb.sh1[j]);
+            tmax = a.w;
+            if (!Single) {
+                scene = &sq.scene(j);
+                nodes = scene->nodes;
+            }
+            return j;
+        },
+        [&](uint32_t j, const S& sl, uint32_t lane) {
+            if (!sl.mark[lane]) sq.deliver(j);
+        });
+}
+
 // ---- ray sorting: a counting sort of the shade output by ray key ------------------------------------------
 // Exclusive scan of the bucket counts into write offsets (one block), then zero the counts. Each warp
 // takes a contiguous 32nd of the buckets and reads it 32 consecutive counts at a time (coalesced):
@@ -1272,6 +1588,27 @@ __global__ void __launch_bounds__(128) k_trace_primary_pairs(const DevScene* sp,
         });
 }
 
+__global__ void __launch_bounds__(128) k_trace_primary_list(const DevScene* sp, CameraArg cam, int w, int h, uint32_t frame, uint32_t seed,
+                                                           float4* out, uint32_t* claim, uint32_t visits) {
+    extern __shared__ int list_smem[];
+    using S = ListSlots<false, true>;
+    S& ls = reinterpret_cast<S*>(list_smem + kListStack * blockDim.x)[threadIdx.x >> 5];
+    const DevScene& s = *sp;
+    const WalkScene uni{s.nodes, s.tris, sp};
+    walk_queue_list<false, true>(
+        uint32_t(w) * uint32_t(h), claim, 24u, visits, list_smem + threadIdx.x, blockDim.x, ls, uni,
+        [&](uint32_t pixel, V3& o, V3& d, float& tmax, const float4*&, const DevScene*&) {
+            const int x = int(pixel % uint32_t(w)), y = int(pixel / uint32_t(w));
+            Rng rng = pixel_rng(pixel, seed, frame);
+            V2 jitter = rng_next2(rng);
+            V2 lens = rng_next2(rng);
+            camera_ray(cam.c, float(x) + jitter.x, float(y) + jitter.y, w, h, lens, o, d);
+            tmax = kInf;
+            return pixel;
+        },
+        [&](uint32_t pixel, const S& sl, uint32_t lane) { out[pixel] = list_hit(sl, lane, sp); });
+}
+
 __global__ void __launch_bounds__(128) k_occlusion_probe_pairs(const DevScene* sp, const float4* rays, int n, int4* out, uint32_t* claim,
                                                               uint32_t visits) {
     extern __shared__ int smem_stack[];
@@ -1404,6 +1741,12 @@ __global__ void k_display(DisplayParams p, const float4* accum, const float4* de
 
 }  // namespace
 
+// A list walk's dynamic shared memory: the block's stacks, then a ListSlots per warp.
+template <bool AnyHit, bool Single>
+static size_t list_smem_bytes(int block) {
+    return size_t(kListStack) * size_t(block) * sizeof(int) + size_t(block / 32) * sizeof(ListSlots<AnyHit, Single>);
+}
+
 cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, LaunchShape* out) {
     cudaDeviceProp prop;
     cudaError_t e = cudaGetDeviceProperties(&prop, device);
@@ -1444,6 +1787,18 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shadow_pairs<false, false, false>, trace_block, pair_smem);
     if (e != cudaSuccess) return e;
     out->pair_shadow_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
+    const void* list_kernels[] = {(const void*)k_trace_list<false>, (const void*)k_trace_list<true>, (const void*)k_shadow_list<false>,
+                                  (const void*)k_shadow_list<true>};
+    for (const void* k : list_kernels) {
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(list_smem_bytes<false, false>(trace_block)));
+        if (e != cudaSuccess) return e;
+    }
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_list<false>, trace_block, list_smem_bytes<false, false>(trace_block));
+    if (e != cudaSuccess) return e;
+    out->list_trace_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shadow_list<false>, trace_block, list_smem_bytes<true, false>(trace_block));
+    if (e != cudaSuccess) return e;
+    out->list_shadow_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     // Grids are sized for the heavier (multi-scene) variants, so that every variant's grid fits.
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace<false, true, false>, trace_block, smem);
     if (e != cudaSuccess) return e;
@@ -1461,6 +1816,11 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
 
 template <bool Count, bool Packed, bool Single>
 static void launch_traversals(const WfParams& p, const LaunchShape& ls, cudaStream_t stream, size_t smem, bool shadow) {
+    if (!Count && Packed && p.pair_visits > 0 && p.order_free && !(shadow && Single && p.wide_shadows)) {
+        if (shadow) k_shadow_list<Single><<<ls.list_shadow_grid, ls.shadow_block, list_smem_bytes<true, Single>(ls.shadow_block), stream>>>(p);
+        else k_trace_list<Single><<<ls.list_trace_grid, ls.trace_block, list_smem_bytes<false, Single>(ls.trace_block), stream>>>(p);
+        return;
+    }
     if (Packed && p.pair_visits > 0) {
         const size_t pair_smem = smem + size_t(ls.trace_block / 32) * sizeof(PairSlots);
         if (shadow && Single && p.wide_shadows) k_shadow_pairs<Count, true, true><<<ls.pair_shadow_grid, ls.shadow_block, pair_smem, stream>>>(p);
@@ -1564,7 +1924,7 @@ cudaError_t wf_accumulate(const DevView* d_view, const DevView& h_view, int firs
 }
 
 cudaError_t wf_trace_primary(const DevScene* scene, const float* cam16, int w, int h, uint32_t frame, uint32_t seed, float4* out,
-                             uint32_t* claim, uint32_t pair_visits, cudaStream_t stream) {
+                             uint32_t* claim, uint32_t pair_visits, bool order_free, cudaStream_t stream) {
     CameraArg c;
     for (int i = 0; i < 16; i++) c.c[i] = cam16[i];
     if (pair_visits > 0) {
@@ -1572,7 +1932,8 @@ cudaError_t wf_trace_primary(const DevScene* scene, const float* cam16, int w, i
         const uint32_t n = uint32_t(w) * uint32_t(h), blocks = std::min<uint32_t>((n + 127) / 128, 148u * 16u);
         cudaError_t e = cudaMemsetAsync(claim, 0, sizeof(uint32_t), stream);
         if (e != cudaSuccess) return e;
-        k_trace_primary_pairs<<<blocks, 128, smem, stream>>>(scene, c, w, h, frame, seed, out, claim, pair_visits);
+        if (order_free) k_trace_primary_list<<<blocks, 128, list_smem_bytes<false, true>(128), stream>>>(scene, c, w, h, frame, seed, out, claim, pair_visits);
+        else k_trace_primary_pairs<<<blocks, 128, smem, stream>>>(scene, c, w, h, frame, seed, out, claim, pair_visits);
         return cudaGetLastError();
     }
     dim3 grid((w + 15) / 16, (h + 7) / 8);

@@ -95,7 +95,10 @@ struct WfParams {
     uint32_t shadow_refill;    // the same for the shadow walk
     uint32_t walk_burst;       // walk steps each lane takes between two looks at its warp (>= 1)
     uint32_t pair_visits;      // > 0: the BVH2 walks are pair walks with up to this many node visits per
-                               //      warp step (packed slab tests only); 0: per-lane walks
+                               //      warp step (packed slab tests only), or list walks (order_free) with
+                               //      twice as many; 0: per-lane walks
+    int order_free;            // 1: every scene of the launch is DevScene::order_free, so that the walks with
+                               //    pair_visits > 0 are list walks (uncounted launches)
     int sort_material;         // 1: the shade kernel groups each block's paths by material class
     int sort_bits;             // > 0: sort continuing paths by direction octant + Morton origin cell
                                //      (this many bits per axis) before they are traced
@@ -121,6 +124,7 @@ struct LaunchShape {
     int shade_grid, shade_block;
     int shadow_grid, shadow_block;
     int pair_trace_grid, pair_shadow_grid;  // the pair walks (more shared memory per block)
+    int list_trace_grid, list_shadow_grid;  // the list walks
 };
 
 // Fills grid sizes from the occupancy of each kernel on `device` (block sizes as requested).
@@ -142,10 +146,10 @@ cudaError_t wf_accumulate(const DevView* d_view, const DevView& h_view, int firs
 // rgb[3i..3i+2] = accum[i].xyz * scale (or the plain xyz when apply_scale is false).
 cudaError_t wf_resolve(const float4* accum, uint32_t n, float scale, bool apply_scale, float* rgb, cudaStream_t stream);
 
-// Probes (same device functions as the wavefront). With pair_visits > 0 the walks are the pair walks
-// of the wavefront's default kernels, over a queue counted in `claim` (one device word).
+// Probes (same device functions as the wavefront). With pair_visits > 0 the walks are the pair walks, or
+// for camera rays of an order-free scene the list walk, over a queue counted in `claim` (one device word).
 cudaError_t wf_trace_primary(const DevScene* scene, const float* cam16, int w, int h, uint32_t frame, uint32_t seed,
-                             float4* out, uint32_t* claim, uint32_t pair_visits, cudaStream_t stream);
+                             float4* out, uint32_t* claim, uint32_t pair_visits, bool order_free, cudaStream_t stream);
 cudaError_t wf_light_picks(const DevScene* scene, const DevView* view, int4* out, int w, int h, cudaStream_t stream);
 cudaError_t wf_heatmap(const DevScene* scene, const float* cam16, int w, int h, float* out, cudaStream_t stream);
 // Any-hit walks of n rays (2 float4 each: origin + tmax, direction + unused): out[i] = (occluded,
