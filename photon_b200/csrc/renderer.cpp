@@ -115,6 +115,9 @@ void WavefrontEngine::reserve_paths(uint64_t needed) {
     keys_.allocate(want);
     shadow_keys_.allocate(want);
     shadow_perm_.allocate(want);
+    order_.allocate(want);
+    classes_.allocate(want);
+    class_ctr_.allocate(128);
     pb_.capacity = uint32_t(want);
     if (graph_) {
         cudaGraphExecDestroy(graph_);
@@ -129,13 +132,14 @@ void WavefrontEngine::release_paths() {
     }
     for (auto& b : bufs_) b.release();
     for (auto& b : ids_) b.release();
-    for (DeviceBuffer<uint32_t>* b : {&keys_, &hist_, &offsets_, &shadow_keys_, &shadow_hist_, &shadow_offsets_, &shadow_perm_}) b->release();
+    for (DeviceBuffer<uint32_t>* b : {&keys_, &hist_, &offsets_, &shadow_keys_, &shadow_hist_, &shadow_offsets_, &shadow_perm_, &order_, &class_ctr_}) b->release();
+    classes_.release();
     pb_ = PathBuffers{};
 }
 
 size_t WavefrontEngine::device_bytes() const {
     size_t b = ctr_.bytes() + keys_.bytes() + hist_.bytes() + offsets_.bytes() + shadow_keys_.bytes() + shadow_hist_.bytes() +
-               shadow_offsets_.bytes() + shadow_perm_.bytes();
+               shadow_offsets_.bytes() + shadow_perm_.bytes() + order_.bytes() + class_ctr_.bytes() + classes_.bytes();
     for (const auto& x : bufs_) b += x.bytes();
     for (const auto& x : ids_) b += x.bytes();
     return b;
@@ -184,6 +188,9 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
     p.packed = tuning_.packed ? 1 : 0;
     p.sort_bits = tuning_.sort_rays;
     p.sort_material = tuning_.sort_by_material;
+    p.order = tuning_.sort_by_material > 0 ? order_.ptr : nullptr;
+    p.classes = classes_.ptr;
+    p.class_ctr = class_ctr_.ptr;
     p.tail_paths = tuning_.tail_paths == kTailAuto ? 1u : uint32_t(std::max(0, tuning_.tail_paths));
     p.wide_shadows = tuning_.wide_shadows;
     p.trace_refill = uint32_t(std::clamp(tuning_.trace_refill, 1, 32));
@@ -251,6 +258,7 @@ void WavefrontEngine::run(const DevScene* scenes, int single_scene, const DevSce
         p.sort_bits = 0;
         p.shadow_sort_bits = 0;
     }
+    if (std::min<uint64_t>(total_work, uint64_t(tuning_.path_capacity)) < kOrderMinPaths) p.order = nullptr;
     bool use_graph = tuning_.graph_bounces > 0;
     bool timed = (profile_flags_ & PT_PROFILE_KERNEL_TIMES) != 0;
     if (use_graph && (!graph_ || std::memcmp(&graph_params_, &p, sizeof(p)) != 0 || graph_iters_ != tuning_.graph_bounces)) capture(p);

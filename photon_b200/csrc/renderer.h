@@ -95,6 +95,8 @@ public:
         cont_params_.sort_bits = on ? tuning_.sort_rays : 0;
         cont_params_.shadow_sort_bits = on ? tuning_.sort_shadows : 0;
     }
+    // Continuous mode: whether the next launches shade in class order over the whole queue.
+    void set_continuous_ordering(bool on) { cont_params_.order = on && tuning_.sort_by_material > 0 ? order_.ptr : nullptr; }
     // Continuous mode: takes the knobs of `t` that only change what the next launches are given
     // (material-sort window, ray-sort bits up to those the buffers were sized for, packed slab tests,
     // 4-wide shadow BVH, walk refill and burst). Pool size, block shapes, graph cadence and the tail
@@ -136,6 +138,8 @@ private:
     DeviceBuffer<uint4> ids_[2];
     DeviceBuffer<Counters> ctr_;
     DeviceBuffer<uint32_t> keys_, hist_, offsets_;
+    DeviceBuffer<uint32_t> order_, class_ctr_;
+    DeviceBuffer<uint8_t> classes_;
     DeviceBuffer<uint32_t> shadow_keys_, shadow_hist_, shadow_offsets_, shadow_perm_;
     Counters* h_ctr_ = nullptr;
     Counters last_{};

@@ -886,6 +886,7 @@ void Server::loop() {
                 const uint32_t tail = engine_->tail_limit_in_use();
                 B.iterations = (tail > 0 && pending <= tail) ? 1 : iters_per_batch_;
                 engine_->set_continuous_sorting(pending >= kSortMinPaths);
+                engine_->set_continuous_ordering(pending >= kOrderMinPaths);
                 PTW_CUDA(cudaEventRecord(B.ev_start, stream_));
                 engine_->launch(B.iterations);
                 batches_++;

@@ -25,6 +25,7 @@ namespace ptw {
 namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
+constexpr uint32_t kShadeKeys = 64;  // shading classes (shade_key)
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
@@ -112,6 +113,8 @@ __device__ __forceinline__ int find_view(const DevView* views, int n, unsigned l
 
 // ---- setup ------------------------------------------------------------------------------------------
 __global__ void k_setup(const __grid_constant__ WfParams P) {
+    if (P.order)
+        for (uint32_t k = threadIdx.x; k < 2 * kShadeKeys; k += blockDim.x) P.class_ctr[k] = 0;
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     Counters* c = P.ctr;
     const uint32_t capacity = P.pb.capacity, tail_paths = P.tail_paths > 0 ? c->tail_limit : 0u;
@@ -884,10 +887,38 @@ __device__ __forceinline__ PathState load_path(const WfParams& P, uint32_t p, ui
     return st;
 }
 
+// A path that left the scene: the environment, weighted against light sampling (integrator.h:159-177),
+// into st.L, and the first vertex's G-buffer.
+__device__ __forceinline__ void shade_miss(const WfParams& P, PathState& st) {
+    const uint4 id = st.id;
+    const DevView& v = P.views[id.x];
+    const DevScene& s = scene_for(P, id.x);
+    const int depth = int(st.flags & 0xffffu);
+    const bool prev_delta = (st.flags >> 16) & 1u;
+    const V3 ro = st.ro, rd = st.rd;
+    V3 le = env_radiance(s, rd);
+    float w = (prev_delta || s.p_env <= 0) ? 1.0f : power_heuristic(st.prev_pdf, env_pdf(s, rd));
+    V3 cc = st.beta * le * w;
+    clamp_contribution(cc, depth, v.clamp);
+    st.L = st.L + cc;
+    if (v.gbuffer && id.w == 0 && depth == 0) {
+        V3 pos = ro + rd * 1e4f;
+        v.g_albedo[id.z] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        v.g_normal_depth[id.z] = make_float4(-rd.x, -rd.y, -rd.z, 0.0f);
+        if (v.g_position) v.g_position[id.z] = make_float4(pos.x, pos.y, pos.z, -1.0f);
+        if (v.g_emission) v.g_emission[id.z] = make_float4(le.x, le.y, le.z, 1.0f);
+        if (v.g_edge) {
+            v.g_edge[id.z] = edge_record(-rd, 0.0f, -1);
+            v.g_motion[id.z] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+}
+
 // One vertex of trace_path for a path whose closest hit is h4 = (t, tri, u, v): adds the emitted
 // light it sees to st.L, writes the first vertex's G-buffer, samples the light (a shadow ray in *sh
 // when `shadow` comes back true) and the continuation (st's ray, throughput and flags). Returns
 // whether the path continues.
+template <bool Misses = true>
 __device__ __forceinline__ bool shade_vertex(const WfParams& P, PathState& st, float4 h4, bool& shadow, ShadowRay& sh) {
     const uint4 id = st.id;
     const DevView& v = P.views[id.x];
@@ -904,24 +935,8 @@ __device__ __forceinline__ bool shade_vertex(const WfParams& P, PathState& st, f
     bool prev_delta = (st.flags >> 16) & 1u;
     int tri = __float_as_int(h4.y);
     bool gbuf = v.gbuffer && id.w == 0 && depth == 0;
-    if (tri < 0) {
-        // Miss: the environment, weighted against light sampling (integrator.h:159-177).
-        V3 le = env_radiance(s, rd);
-        float w = (prev_delta || s.p_env <= 0) ? 1.0f : power_heuristic(prev_pdf, env_pdf(s, rd));
-        V3 cc = beta * le * w;
-        clamp_contribution(cc, depth, v.clamp);
-        L = L + cc;
-        if (gbuf) {
-            V3 pos = ro + rd * 1e4f;
-            v.g_albedo[id.z] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
-            v.g_normal_depth[id.z] = make_float4(-rd.x, -rd.y, -rd.z, 0.0f);
-            if (v.g_position) v.g_position[id.z] = make_float4(pos.x, pos.y, pos.z, -1.0f);
-            if (v.g_emission) v.g_emission[id.z] = make_float4(le.x, le.y, le.z, 1.0f);
-            if (v.g_edge) {
-                v.g_edge[id.z] = edge_record(-rd, 0.0f, -1);
-                v.g_motion[id.z] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-        }
+    if (Misses && tri < 0) {
+        shade_miss(P, st);
         return false;
     }
     Interaction it = surface_at(s, ro, rd, h4.x, tri, h4.z, h4.w);
@@ -996,8 +1011,21 @@ __device__ __forceinline__ bool shade_vertex(const WfParams& P, PathState& st, f
     return cont;
 }
 
+// Progress of views that count finished paths (the request server); every lane of the warp calls it.
+__device__ __forceinline__ void count_finished(const WfParams& P, bool finished, uint32_t view) {
+    if (P.num_views > 1 || P.views[0].done_counter) {
+        uint32_t key = finished ? view : 0xffffffffu;
+        uint32_t peers = __match_any_sync(kFull, key);
+        if (finished && int(lane_id()) == __ffs(peers) - 1) {
+            unsigned long long* dc = P.views[view].done_counter;
+            if (dc) atomicAdd(dc, (unsigned long long)__popc(peers));
+        }
+    }
+}
+
 // Shades path `i` of the current queue and appends its continuation and shadow ray to the next
 // queues (every lane of the warp calls it; `active` is false for lanes without a path).
+template <bool Misses>
 __device__ __forceinline__ void shade_path(const WfParams& P, Counters* c, uint32_t p, uint32_t i, bool active) {
     const uint32_t q = p ^ 1u;
     bool cont = false, shadow = false;
@@ -1005,7 +1033,7 @@ __device__ __forceinline__ void shade_path(const WfParams& P, Counters* c, uint3
     ShadowRay sh;
     if (active) {
         st = load_path(P, p, i);
-        cont = shade_vertex(P, st, P.pb.hit[i], shadow, sh);
+        cont = shade_vertex<Misses>(P, st, P.pb.hit[i], shadow, sh);
     } else {
         st.id = make_uint4(0, 0, 0, 0);
     }
@@ -1046,21 +1074,11 @@ __device__ __forceinline__ void shade_path(const WfParams& P, Counters* c, uint3
         P.pb.sh1[qs] = make_float4(sh.d.x, sh.d.y, sh.d.z, __uint_as_float(cont ? slot : id.y));
         P.pb.sh2[qs] = make_float4(sh.c.x, sh.c.y, sh.c.z, __uint_as_float(id.x | (cont ? 0u : 0x80000000u)));
     }
-    // Progress of views that count finished paths (the request server).
-    bool finished = active && !cont;
-    if (P.num_views > 1 || P.views[0].done_counter) {
-        uint32_t key = finished ? id.x : 0xffffffffu;
-        uint32_t peers = __match_any_sync(kFull, key);
-        if (finished && int(lane_id()) == __ffs(peers) - 1) {
-            unsigned long long* dc = P.views[id.x].done_counter;
-            if (dc) atomicAdd(dc, (unsigned long long)__popc(peers));
-        }
-    }
+    count_finished(P, active && !cont, id.x);
 }
 
 // The shading class of a queued path: 0 for a miss, else the class of the hit triangle's material
 // (1..32, precomputed per material at upload from its lobes, textures and emission).
-constexpr uint32_t kShadeKeys = 64;
 __device__ __forceinline__ uint32_t shade_key(const WfParams& P, uint32_t p, uint32_t i) {
     int tri = __float_as_int(P.pb.hit[i].y);
     if (tri < 0) return 0;
@@ -1068,8 +1086,8 @@ __device__ __forceinline__ uint32_t shade_key(const WfParams& P, uint32_t p, uin
     return s.shade_keys[__float_as_int(__ldg(s.tris + kTriStride * tri).w)];
 }
 
-// Persistent over the queue. Without material sorting each warp claims 32 paths in queue order. With
-// it each block claims a window of sort_material x blockDim paths, orders them by shading class in
+// Small renders' shading. Persistent over the queue. Without material sorting each warp claims 32 paths in
+// queue order. With it each block claims a window of sort_material x blockDim paths, orders them by shading class in
 // shared memory (a counting sort on 64 keys) and shades them in that order, so a warp mostly runs one
 // BSDF lobe and one texture pattern. The order in which paths are shaded changes only where their
 // outputs are appended, not any path's result.
@@ -1087,7 +1105,7 @@ __global__ void __launch_bounds__(256) k_shade(const __grid_constant__ WfParams 
             uint32_t i0 = warp_fetch(&c->fetch[2]);
             if (i0 >= n) break;
             uint32_t i = i0 + lane_id();
-            shade_path(P, c, p, i, i < n);
+            shade_path<true>(P, c, p, i, i < n);
         }
         return;
     }
@@ -1138,9 +1156,135 @@ __global__ void __launch_bounds__(256) k_shade(const __grid_constant__ WfParams 
         __syncthreads();
         for (uint32_t r = 0; r < rounds; r++) {
             const uint32_t j = s_perm[r * blockDim.x + tid];
-            shade_path(P, c, p, j, j < n);
+            shade_path<true>(P, c, p, j, j < n);
         }
         __syncthreads();
+    }
+}
+
+// ---- shading in class order ------------------------------------------------------------------------------
+// Renders of at least kOrderMinPaths paths are shaded in the order of their shading classes over the whole
+// queue: a counting sort (k_class_count, k_class_order) writes the order, k_shade_misses takes the paths
+// that left the scene and k_shade_ordered the others, without a block barrier. Against windows ordered in
+// the shade kernel itself (k_shade) this takes out what that kernel waited for besides its gathers: per
+// issued instruction of 15 cycles it stalled 1.7-3.3 at the windows' barriers and 3.1-4.0 for instructions
+// (its blocks run all classes' code at once, which does not fit the instruction caches; in class order the
+// whole chip runs one class at a time), and its window keys, a dependent gather at 16 warps per SM, were
+// 14% of its time. The order in which paths are shaded changes only where their outputs are appended.
+// 1080p frame of the 262K scene, all shading: 11.1 -> 7.4 ms (7.6 with the misses in k_shade_ordered);
+// 1.05M triangles, 720p at 8 spp: 3.25 -> 2.05; the box at 256x256, 64 spp: 2.04 -> 1.83. Of one 2.07M-path
+// iteration: count 23 us, order 14, misses 28, the hits 224 (windows: 409 in all). At 230,000 paths both
+// ways take the same; a smaller render keeps k_shade, whose single launch is cheaper.
+constexpr uint32_t kClassTile = 2048;  // paths of a block's tile, eight per thread
+__global__ void __launch_bounds__(256) k_class_count(const __grid_constant__ WfParams P) {
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t p = c->parity, n = c->count[p], tid = threadIdx.x;
+    __shared__ uint32_t s_hist[kShadeKeys];
+    for (uint32_t k = tid; k < kShadeKeys; k += blockDim.x) s_hist[k] = 0;
+    __syncthreads();
+    for (uint32_t i0 = blockIdx.x * kClassTile; i0 < n; i0 += gridDim.x * kClassTile) {
+        uint32_t key[8];
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            const uint32_t i = i0 + q * 256 + tid;
+            key[q] = i < n ? shade_key(P, p, i) : kShadeKeys;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            const uint32_t i = i0 + q * 256 + tid;
+            // Misses, about half of the paths, as one addition per warp.
+            const uint32_t miss = __ballot_sync(kFull, key[q] == 0);
+            if (key[q] == 0) {
+                if (int(lane_id()) == __ffs(miss) - 1) atomicAdd(&s_hist[0], uint32_t(__popc(miss)));
+            } else if (key[q] < kShadeKeys) {
+                atomicAdd(&s_hist[key[q]], 1u);
+            }
+            if (i < n) P.classes[i] = uint8_t(key[q]);
+        }
+    }
+    __syncthreads();
+    if (tid < kShadeKeys && s_hist[tid]) atomicAdd(&P.class_ctr[tid], s_hist[tid]);
+}
+
+__global__ void __launch_bounds__(256) k_class_order(const __grid_constant__ WfParams P) {
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t n = c->count[c->parity], tid = threadIdx.x;
+    __shared__ uint32_t s_first[kShadeKeys], s_hist[kShadeKeys], s_base[kShadeKeys];
+    if (tid < 32) {  // exclusive scan of the 64 class counts, two per lane
+        const uint32_t a = P.class_ctr[2 * tid], b = P.class_ctr[2 * tid + 1];
+        uint32_t incl = a + b;
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, incl, off);
+            if (int(tid) >= off) incl += v;
+        }
+        s_first[2 * tid] = incl - a - b;
+        s_first[2 * tid + 1] = incl - b;
+    }
+    for (uint32_t i0 = blockIdx.x * kClassTile; i0 < n; i0 += gridDim.x * kClassTile) {
+        __syncthreads();
+        if (tid < kShadeKeys) s_hist[tid] = 0;
+        __syncthreads();
+        uint32_t key[8], rank[8];
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            const uint32_t i = i0 + q * 256 + tid;
+            key[q] = i < n ? P.classes[i] : kShadeKeys;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++) {
+            const uint32_t miss = __ballot_sync(kFull, key[q] == 0);
+            rank[q] = 0;
+            if (key[q] == 0) {
+                const int leader = __ffs(miss) - 1;
+                uint32_t base = 0;
+                if (int(lane_id()) == leader) base = atomicAdd(&s_hist[0], uint32_t(__popc(miss)));
+                rank[q] = __shfl_sync(miss, base, leader) + uint32_t(__popc(miss & ((1u << lane_id()) - 1u)));
+            } else if (key[q] < kShadeKeys) {
+                rank[q] = atomicAdd(&s_hist[key[q]], 1u);
+            }
+        }
+        __syncthreads();
+        if (tid < kShadeKeys) s_base[tid] = s_first[tid] + (s_hist[tid] ? atomicAdd(&P.class_ctr[kShadeKeys + tid], s_hist[tid]) : 0u);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t q = 0; q < 8; q++)
+            if (key[q] < kShadeKeys) P.order[s_base[key[q]] + rank[q]] = i0 + q * 256 + tid;
+    }
+}
+
+// The misses, class 0 and first in the order, about half of an open scene's paths: bound by the path
+// state's bandwidth, so they get a kernel of few registers (46: five blocks of 256 threads per SM).
+__global__ void __launch_bounds__(256) k_shade_misses(const __grid_constant__ WfParams P) {
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t p = c->parity, n = P.class_ctr[0];
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t i0 = (blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * 32u; i0 < n; i0 += warps * 32u) {
+        const uint32_t i = i0 + lane_id();
+        const bool active = i < n;
+        uint32_t view = 0;
+        if (active) {
+            PathState st = load_path(P, p, P.order[i]);
+            shade_miss(P, st);
+            view = st.id.x;
+            P.views[view].sample_out[st.id.y] = make_float4(st.L.x, st.L.y, st.L.z, 0.0f);
+        }
+        count_finished(P, active, view);
+    }
+}
+
+// The hits. 96 registers without spills, 20 warps per SM (24 with 80 registers spill: 7.5 ms against 7.4);
+// bound by the latency of its gathers. (Prefetching the next paths' state into L1 changed nothing.)
+__global__ void __launch_bounds__(128, 5) k_shade_ordered(const __grid_constant__ WfParams P) {
+    Counters* c = P.ctr;
+    if (c->tail) return;
+    const uint32_t p = c->parity, n = c->count[p];
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    for (uint32_t i0 = P.class_ctr[0] + (blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u) * 32u; i0 < n; i0 += warps * 32u) {
+        const uint32_t i = i0 + lane_id();
+        shade_path<false>(P, c, p, i < n ? P.order[i] : 0u, i < n);
     }
 }
 
@@ -1811,6 +1955,12 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade, shade_block, 0);
     if (e != cudaSuccess) return e;
     out->shade_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade_ordered, 128, 0);
+    if (e != cudaSuccess) return e;
+    out->ordered_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade_misses, 256, 0);
+    if (e != cudaSuccess) return e;
+    out->misses_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     return cudaSuccess;
 }
 
@@ -1880,7 +2030,14 @@ cudaError_t wf_iteration(const WfParams& p, const LaunchShape& ls, cudaStream_t 
     if (p.tail_paths > 0) launch_tail(p, ls, stream, smem);
     launch_traversal(p, ls, stream, smem, false);
     mark(3);
-    k_shade<<<ls.shade_grid, ls.shade_block, 0, stream>>>(p);
+    if (p.order) {
+        k_class_count<<<ls.gen_grid, 256, 0, stream>>>(p);
+        k_class_order<<<ls.gen_grid, 256, 0, stream>>>(p);
+        k_shade_misses<<<ls.misses_grid, 256, 0, stream>>>(p);
+        k_shade_ordered<<<ls.ordered_grid, 128, 0, stream>>>(p);
+    } else {
+        k_shade<<<ls.shade_grid, ls.shade_block, 0, stream>>>(p);
+    }
     mark(4);
     if (p.shadow_sort_bits > 0) {
         k_sort_scan<true><<<1, 1024, 0, stream>>>(p, 8u << (3 * p.shadow_sort_bits));

@@ -100,6 +100,9 @@ struct WfParams {
     int order_free;            // 1: every scene of the launch is DevScene::order_free, so that the walks with
                                //    pair_visits > 0 are list walks (uncounted launches)
     int sort_material;         // 1: the shade kernel groups each block's paths by material class
+    uint32_t* order;           // capacity entries: the shade order by class, or null (shaded by k_shade)
+    uint8_t* classes;          // capacity entries: their shading classes
+    uint32_t* class_ctr;       // per class: paths of the iteration, then paths placed in the order
     int sort_bits;             // > 0: sort continuing paths by direction octant + Morton origin cell
                                //      (this many bits per axis) before they are traced
     uint32_t* keys;            // capacity entries (sort keys of the shade output)
@@ -125,6 +128,7 @@ struct LaunchShape {
     int shadow_grid, shadow_block;
     int pair_trace_grid, pair_shadow_grid;  // the pair walks (more shared memory per block)
     int list_trace_grid, list_shadow_grid;  // the list walks
+    int ordered_grid, misses_grid;          // shading in class order
 };
 
 // Fills grid sizes from the occupancy of each kernel on `device` (block sizes as requested).
@@ -136,9 +140,11 @@ cudaError_t wf_iteration(const WfParams& p, const LaunchShape& ls, cudaStream_t 
 // Iterations with fewer queued paths are not ray-sorted (the scan and scatter would cost more than the
 // coherence gains).
 constexpr uint32_t kSortMinPaths = 1u << 21;
+// Renders of fewer paths are not shaded in class order over the whole queue.
+constexpr uint32_t kOrderMinPaths = 1u << 18;
 // Kernels wf_iteration launches for these parameters.
 inline int wf_kernels_per_iteration(const WfParams& p) {
-    return 5 + (p.tail_paths > 0 ? 1 : 0) + (p.sort_bits > 0 ? 3 : 0) + (p.shadow_sort_bits > 0 ? 2 : 0);
+    return 5 + (p.order ? 3 : 0) + (p.tail_paths > 0 ? 1 : 0) + (p.sort_bits > 0 ? 3 : 0) + (p.shadow_sort_bits > 0 ? 2 : 0);
 }
 // Sums the samples of every pixel of a view in sample order (after a pass).
 cudaError_t wf_accumulate(const DevView* d_view, const DevView& h_view, int first_pass, int last_pass, cudaStream_t stream);
