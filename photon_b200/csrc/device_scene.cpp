@@ -90,7 +90,7 @@ size_t DeviceScene::device_bytes() const {
     return nodes_.bytes() + nodes4_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
            punctual_.bytes() + env_texels_.bytes() + tri_idx_.bytes() + textures_.bytes() + uvs_.bytes() + texels_.bytes() +
            srgb_lut_.bytes() + env_marginal_.bytes() + env_conditional_.bytes() + env_row_sin_.bytes() + emissive_.bytes() +
-           shade_keys_.bytes() + d_view_.bytes();
+           shade_keys_.bytes() + light_work_.bytes() + d_view_.bytes();
 }
 
 // Shading classes: materials of one class take the same branches through the BSDF, texture and

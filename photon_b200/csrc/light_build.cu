@@ -7,6 +7,7 @@
 // in the host's order.
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -157,41 +158,118 @@ __global__ void k_env_texels(const float* __restrict__ rgb, size_t n, float4* __
     out[i] = make_float4(x, y, z, lum3(x, y, z));
 }
 
-__global__ void k_env_rows(const float4* __restrict__ texels, int w, int h, const float* __restrict__ row_sin, float* __restrict__ cond,
-                           double* __restrict__ row_total) {
-    const int y = blockIdx.x * blockDim.x + threadIdx.x;
-    if (y >= h) return;
+// Each row's conditional CDF, a block per row. The prefix sums are the host's, in its order: the block
+// forms a tile's terms in parallel, one thread chains them, and the divisions are parallel again (one
+// thread per row for everything, with its strided reads, took 0.9 ms for a 1024x512 image; this takes 0.05).
+constexpr int kRowTile = 1024;
+__global__ void __launch_bounds__(128) k_env_rows(const float4* __restrict__ texels, int w, int h, const float* __restrict__ row_sin,
+                                                  float* __restrict__ cond, double* __restrict__ row_total) {
+    __shared__ double term[kRowTile];
+    const int y = blockIdx.x;
     const float sin_theta = row_sin[y];
     const float4* row = texels + size_t(y) * size_t(w);
-    double rs = 0;
-    for (int x = 0; x < w; x++) rs = rs + double(row[x].w) * sin_theta;
-    row_total[y] = rs;
     float* cdf = cond + size_t(y) * size_t(w + 1);
-    cdf[0] = 0.0f;
-    double prefix = 0;
-    for (int x = 1; x <= w; x++) {
-        prefix = prefix + double(row[x - 1].w) * sin_theta;
-        cdf[x] = rs > 0 ? float(double(float(prefix)) / rs) : float(x) / float(w);
+    double prefix = 0;  // thread 0's
+    for (int x0 = 0; x0 < w; x0 += kRowTile) {
+        const int n = min(kRowTile, w - x0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) term[k] = double(row[x0 + k].w) * sin_theta;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < n; k++) {
+                prefix = prefix + term[k];
+                term[k] = prefix;
+            }
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) cdf[x0 + k + 1] = float(term[k]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        term[0] = prefix;
+        row_total[y] = prefix;
+        cdf[0] = 0.0f;
+    }
+    __syncthreads();
+    const double rs = term[0];
+    for (int x = 1 + int(threadIdx.x); x <= w; x += blockDim.x) cdf[x] = rs > 0 ? float(double(cdf[x]) / rs) : float(x) / float(w);
+}
+
+// The marginal CDF and the integral: the row sums chained by one thread, the divisions in parallel.
+__global__ void __launch_bounds__(256) k_env_marginal(int w, int h, const double* __restrict__ row_total, float* __restrict__ marginal,
+                                                      float* __restrict__ scalars) {
+    __shared__ double total;
+    __shared__ double term[kRowTile];
+    double all = 0;  // thread 0's
+    for (int y0 = 0; y0 < h; y0 += kRowTile) {
+        const int n = min(kRowTile, h - y0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) term[k] = row_total[y0 + k];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < n; k++) {
+                all = all + term[k];
+                term[k] = all;
+            }
+        __syncthreads();
+        for (int k = threadIdx.x; k < n; k += blockDim.x) marginal[y0 + k + 1] = float(term[k]);
+    }
+    if (threadIdx.x == 0) {
+        total = all;
+        marginal[0] = 0.0f;
+        scalars[0] = float(all / (double(w) * double(h)));
+    }
+    __syncthreads();
+    all = total;
+    for (int y = 1 + int(threadIdx.x); y <= h; y += blockDim.x) marginal[y] = all > 0 ? float(double(marginal[y]) / all) : float(y) / float(h);
+}
+
+// Sums of the texels' luminances and of their absolute values, in any order (k_env_mean).
+__global__ void __launch_bounds__(256) k_env_sums(const float4* __restrict__ texels, size_t n, double* __restrict__ sums) {
+    double s = 0, a = 0;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+        const double l = texels[i].w;
+        s += l;
+        a += fabs(l);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(sums, s);
+        atomicAdd(sums + 1, a);
     }
 }
 
-// The marginal CDF, the integral and the mean luminance (one thread, the host's order).
-__global__ void k_env_marginal(const float4* __restrict__ texels, int w, int h, const double* __restrict__ row_total,
-                               float* __restrict__ marginal, float* __restrict__ scalars) {
+// The mean luminance as the host rounds it: the float nearest to (the sum in texel order) / n. Any two
+// orders of n double additions differ by at most 2 n u sum |l| (u = 2^-53), so when both ends of that
+// interval round to one float, it is the host's; otherwise (about one image in 500) one thread takes the
+// sum in order. That chain, which was the whole of it, is 13 ms for a 1024x512 image.
+__global__ void k_env_mean(const float4* __restrict__ texels, size_t n, const double* __restrict__ sums, float* __restrict__ scalars) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double all = 0;
-    marginal[0] = 0.0f;
-    for (int y = 0; y < h; y++) {
-        all = all + row_total[y];
-        marginal[y + 1] = float(all);  // the prefix, normalised below
+    const double slack = 2.1 * double(n) * 0x1p-53 * sums[1];
+    const float lo = float((sums[0] - slack) / double(n)), hi = float((sums[0] + slack) / double(n));
+    if (lo == hi && isfinite(lo)) {
+        scalars[1] = lo;
+        return;
     }
-    for (int y = 1; y <= h; y++) marginal[y] = all > 0 ? float(double(marginal[y]) / all) : float(y) / float(h);
-    scalars[0] = float(all / (double(w) * double(h)));
     double s = 0;
-    const size_t n = size_t(w) * size_t(h);
     for (size_t i = 0; i < n; i++) s += texels[i].w;
     scalars[1] = float(s / double(n));
 }
+
+// Hands out 256-byte aligned pieces of a buffer; over a null buffer it only adds up their sizes.
+struct Carver {
+    uint8_t* base;
+    size_t used = 0;
+    explicit Carver(uint8_t* b) : base(b) {}
+    template <typename T>
+    T* take(size_t n) {
+        T* p = reinterpret_cast<T*>(base + used);
+        used += (n * sizeof(T) + 255) / 256 * 256;
+        return p;
+    }
+};
 
 float lum_h(const pt_vec3& c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
 
@@ -213,61 +291,73 @@ void DeviceScene::rebuild_lights(const pt_light_update& u, cudaStream_t s) {
     const int n = view_.num_tris;
     materials_.upload(reinterpret_cast<const float4*>(u.materials), size_t(u.num_materials) * 5, s);
     upload_shade_keys(u.materials, u.num_materials, s);
+    // The call's scratch, carved out of one buffer that stays with the scene (a dozen allocations and
+    // frees per call took about 2 ms).
+    const bool has_env_image = u.env_texels != nullptr;
+    const size_t env_n = has_env_image ? size_t(u.env_width) * size_t(u.env_height) : 0, m1 = size_t(n) + 1;
+    size_t scan_bytes = 0;
+    PTW_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, static_cast<int*>(nullptr), static_cast<int*>(nullptr), n + 1, s));
+    Carver size(nullptr);
+    int *flag = nullptr, *pos = nullptr, *under = nullptr, *over = nullptr;
+    float *area = nullptr, *power = nullptr, *power_c = nullptr, *scalars = nullptr, *rgb = nullptr;
+    double *fill = nullptr, *row_total = nullptr, *sums = nullptr;
+    uint8_t* scan_temp = nullptr;
+    auto carve = [&](Carver& c) {
+        // (The emitters are at most the triangles.)
+        fill = c.take<double>(m1);
+        row_total = c.take<double>(has_env_image ? size_t(u.env_height) : 0);
+        sums = c.take<double>(2);
+        flag = c.take<int>(m1);
+        pos = c.take<int>(m1);
+        under = c.take<int>(m1);
+        over = c.take<int>(m1);
+        area = c.take<float>(m1);
+        power = c.take<float>(m1);
+        power_c = c.take<float>(m1);
+        scalars = c.take<float>(4);
+        rgb = c.take<float>(3 * env_n);
+        scan_temp = c.take<uint8_t>(scan_bytes + 1);
+    };
+    carve(size);
+    light_work_.reserve(size.used);
+    Carver work(light_work_.ptr);
+    carve(work);
     // Emissive triangles, in triangle order.
-    DeviceBuffer<int> flag, pos;
-    DeviceBuffer<float> area, power, power_c;
-    flag.allocate(size_t(n) + 1);
-    pos.allocate(size_t(n) + 1);
-    area.allocate(size_t(n) + 1);
-    power.allocate(size_t(n) + 1);
     TexArgs T{textures_.ptr, texels_.ptr, srgb_lut_.ptr, num_textures};
     int ne = 0;
     if (n > 0) {
-        k_light_tris<<<(n + 255) / 256, 256, 0, s>>>(materials_.ptr, tris_.ptr, tri_idx_.ptr, uvs_.ptr, T, n, flag.ptr, area.ptr, power.ptr);
+        k_light_tris<<<(n + 255) / 256, 256, 0, s>>>(materials_.ptr, tris_.ptr, tri_idx_.ptr, uvs_.ptr, T, n, flag, area, power);
         PTW_CUDA(cudaGetLastError());
-        size_t temp = 0;
-        PTW_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, flag.ptr, pos.ptr, n + 1, s));
-        DeviceBuffer<uint8_t> tmp;
-        tmp.allocate(temp + 1);
-        PTW_CUDA(cudaMemsetAsync(flag.ptr + n, 0, sizeof(int), s));
-        PTW_CUDA(cub::DeviceScan::ExclusiveSum(tmp.ptr, temp, flag.ptr, pos.ptr, n + 1, s));
-        PTW_CUDA(cudaMemcpyAsync(&ne, pos.ptr + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+        PTW_CUDA(cudaMemsetAsync(flag + n, 0, sizeof(int), s));
+        PTW_CUDA(cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, flag, pos, n + 1, s));
+        PTW_CUDA(cudaMemcpyAsync(&ne, pos + n, sizeof(int), cudaMemcpyDeviceToHost, s));
         PTW_CUDA(cudaStreamSynchronize(s));
     }
     emissive_.allocate(size_t(ne));
     alias_.allocate(size_t(ne));
-    power_c.allocate(size_t(ne) + 1);
     if (n > 0) {
-        k_light_scatter<<<(n + 255) / 256, 256, 0, s>>>(flag.ptr, pos.ptr, area.ptr, power.ptr, n, tri_idx_.ptr, emissive_.ptr, power_c.ptr);
+        k_light_scatter<<<(n + 255) / 256, 256, 0, s>>>(flag, pos, area, power, n, tri_idx_.ptr, emissive_.ptr, power_c);
         PTW_CUDA(cudaGetLastError());
     }
-    DeviceBuffer<double> fill;
-    DeviceBuffer<int> under, over;
-    DeviceBuffer<float> scalars;
-    fill.allocate(size_t(ne) + 1);
-    under.allocate(size_t(ne) + 1);
-    over.allocate(size_t(ne) + 1);
-    scalars.allocate(4);
-    k_light_alias<<<1, 32, 0, s>>>(power_c.ptr, ne, alias_.ptr, fill.ptr, under.ptr, over.ptr, scalars.ptr + 2);
+    k_light_alias<<<1, 32, 0, s>>>(power_c, ne, alias_.ptr, fill, under, over, scalars + 2);
     PTW_CUDA(cudaGetLastError());
     // Environment.
-    const bool has_env_image = u.env_texels != nullptr;
     if (has_env_image) {
         const int w = u.env_width, h = u.env_height;
-        const size_t texn = size_t(w) * size_t(h);
-        DeviceBuffer<float> rgb;
-        rgb.upload(reinterpret_cast<const float*>(u.env_texels), 3 * texn, s);
+        const size_t texn = env_n;
+        PTW_CUDA(cudaMemcpyAsync(rgb, u.env_texels, 3 * texn * sizeof(float), cudaMemcpyHostToDevice, s));
         env_texels_.allocate(texn);
-        k_env_texels<<<unsigned((texn + 255) / 256), 256, 0, s>>>(rgb.ptr, texn, env_texels_.ptr);
+        k_env_texels<<<unsigned((texn + 255) / 256), 256, 0, s>>>(rgb, texn, env_texels_.ptr);
         std::vector<float> row_sin(static_cast<size_t>(h));
         for (int y = 0; y < h; y++) row_sin[size_t(y)] = std::sin((float(y) + 0.5f) / float(h) * kPiF);
         env_row_sin_.upload(row_sin.data(), row_sin.size(), s);
         env_conditional_.allocate(size_t(h) * size_t(w + 1));
         env_marginal_.allocate(size_t(h) + 1);
-        DeviceBuffer<double> row_total;
-        row_total.allocate(size_t(h));
-        k_env_rows<<<(h + 127) / 128, 128, 0, s>>>(env_texels_.ptr, w, h, env_row_sin_.ptr, env_conditional_.ptr, row_total.ptr);
-        k_env_marginal<<<1, 32, 0, s>>>(env_texels_.ptr, w, h, row_total.ptr, env_marginal_.ptr, scalars.ptr);
+        PTW_CUDA(cudaMemsetAsync(sums, 0, 2 * sizeof(double), s));
+        k_env_rows<<<h, 128, 0, s>>>(env_texels_.ptr, w, h, env_row_sin_.ptr, env_conditional_.ptr, row_total);
+        k_env_marginal<<<1, 256, 0, s>>>(w, h, row_total, env_marginal_.ptr, scalars);
+        k_env_sums<<<unsigned(std::min<size_t>((texn + 255) / 256, 592)), 256, 0, s>>>(env_texels_.ptr, texn, sums);
+        k_env_mean<<<1, 32, 0, s>>>(env_texels_.ptr, texn, sums, scalars);
         PTW_CUDA(cudaGetLastError());
         PTW_CUDA(cudaStreamSynchronize(s));
     } else {
@@ -277,7 +367,7 @@ void DeviceScene::rebuild_lights(const pt_light_update& u, cudaStream_t s) {
         env_row_sin_.release();
     }
     float sc[4] = {0, 0, 0, 0};
-    PTW_CUDA(cudaMemcpyAsync(sc, scalars.ptr, sizeof(sc), cudaMemcpyDeviceToHost, s));
+    PTW_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(sc), cudaMemcpyDeviceToHost, s));
     punctual_.upload(reinterpret_cast<const float4*>(u.punctual), size_t(u.num_punctual) * 3, s);
     PTW_CUDA(cudaStreamSynchronize(s));
     const float env_integral = has_env_image ? sc[0] : 0.0f;
