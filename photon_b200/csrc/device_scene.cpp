@@ -8,6 +8,7 @@
 #include "device_scene.h"
 #include "tree_check.h"
 #include "wide_bvh.h"
+#include "wide_tree.h"
 
 #include <algorithm>
 #include <cmath>
@@ -78,7 +79,7 @@ void validate_scene(const pt_scene_desc& d, bool lights_only) {
 
 size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
     size_t b = 0;
-    b += size_t(d.num_nodes) * 64 + size_t(d.num_tris) * (16 * kTriStride + 16);
+    b += size_t(d.num_nodes) * (64 + 96) + size_t(d.num_tris) * (16 * kTriStride + 16);
     b += size_t(d.num_vertices) * ((d.normals ? 16 : 0) + (d.uvs ? 8 : 0) + (d.tangents ? 16 : 0));
     b += size_t(d.num_materials) * 80 + size_t(d.num_textures) * 16 + size_t(d.num_texels) * 4 + 1024;
     b += size_t(d.num_emissive) * 24 + size_t(d.num_punctual) * 48;
@@ -87,7 +88,7 @@ size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
 }
 
 size_t DeviceScene::device_bytes() const {
-    return nodes_.bytes() + nodes4_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
+    return nodes_.bytes() + nodes4_.bytes() + wide_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
            punctual_.bytes() + env_texels_.bytes() + tri_idx_.bytes() + textures_.bytes() + uvs_.bytes() + texels_.bytes() +
            srgb_lut_.bytes() + env_marginal_.bytes() + env_conditional_.bytes() + env_row_sin_.bytes() + emissive_.bytes() +
            shade_keys_.bytes() + light_work_.bytes() + d_view_.bytes();
@@ -246,6 +247,17 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
     v.bvh_depth = tree_depth_;
     v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_depth_, s) ? 1 : 0;
+    if (!v.order_free) {
+        wide_.release();
+    } else if (!lights_only || !wide_.ptr) {
+        DeviceBuffer<float4> room;
+        room.allocate(size_t(v.num_nodes) * 2 * kWide);
+        const int n = wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, room.ptr, s);
+        wide_.allocate(size_t(n) * 2 * kWide);
+        PTW_CUDA(cudaMemcpyAsync(wide_.ptr, room.ptr, wide_.bytes(), cudaMemcpyDeviceToDevice, s));
+        PTW_CUDA(cudaStreamSynchronize(s));
+    }
+    v.wide = wide_.ptr;
     {
         float lo[3] = {d.bounds_min.x, d.bounds_min.y, d.bounds_min.z}, hi[3] = {d.bounds_max.x, d.bounds_max.y, d.bounds_max.z};
         float inv[3];

@@ -89,7 +89,7 @@ public:
     void rebuild_lights(const pt_light_update& u, cudaStream_t stream);
 
 private:
-    DeviceBuffer<float4> nodes4_;
+    DeviceBuffer<float4> nodes4_, wide_;
     DeviceBuffer<float4> nodes_, tris_, normals_, tangents_, materials_, alias_, punctual_, env_texels_;
     DeviceBuffer<int4> tri_idx_, textures_;
     DeviceBuffer<float2> uvs_;

@@ -23,6 +23,7 @@ constexpr int kTriStride = 4;
 struct DevScene {
     const float4* nodes;
     const float4* nodes4;     // the 4-wide BVH for any-hit rays (8 float4 per node), or null
+    const float4* wide;       // the group walk's 8-wide tree (wide_tree.h), or null unless order_free
     const float4* tris;
     const int4* tri_idx;
     const float4* normals;

@@ -31,9 +31,12 @@ struct RenderCount {
     }
 };
 
-uint32_t tail_limit(int tail_paths, bool alone) {
-    if (tail_paths == kTailAuto) return uint32_t(alone ? kTailAlone : kTailShared);
-    return tail_paths > 0 ? uint32_t(tail_paths) : 0u;
+// The tail's threshold for a render beside `others` on the device; `group`: its tail walks rays by groups;
+// `small`: over a tree of few nodes, whose rays are short.
+uint32_t tail_limit(int tail_paths, bool group, bool small, int others) {
+    if (tail_paths != kTailAuto) return tail_paths > 0 ? uint32_t(tail_paths) : 0u;
+    if (group) return uint32_t(others == 0 && !small ? kGroupTailAlone : others <= 2 ? kGroupTailFew : kGroupTailMany);
+    return uint32_t(others == 0 ? kTailAlone : kTailShared);
 }
 
 }  // namespace
@@ -193,6 +196,7 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
     p.class_ctr = class_ctr_.ptr;
     p.tail_paths = tuning_.tail_paths == kTailAuto ? 1u : uint32_t(std::max(0, tuning_.tail_paths));
     p.wide_shadows = tuning_.wide_shadows;
+    p.group_tail = p.order_free && !count && tuning_.packed && tuning_.pair_walk > 0 ? kGroupTail : 0u;
     p.trace_refill = uint32_t(std::clamp(tuning_.trace_refill, 1, 32));
     p.shadow_refill = uint32_t(std::clamp(tuning_.shadow_refill, 1, 32));
     p.walk_burst = uint32_t(std::clamp(tuning_.walk_burst, 1, 1 << 20));
@@ -250,9 +254,9 @@ void WavefrontEngine::run(const DevScene* scenes, int single_scene, const DevSce
     std::memset(h_ctr_, 0, sizeof(Counters));
     h_ctr_->parity = 1;
     h_ctr_->work_total = total_work;
-    h_ctr_->tail_limit = tail_limit(tuning_.tail_paths, busy.others == 0);
-    PTW_CUDA(cudaMemcpyAsync(ctr_.ptr, h_ctr_, sizeof(Counters), cudaMemcpyHostToDevice, stream_));
     WfParams p = params(scenes, single_scene, single, views, n_views, count_work || (profile_flags_ & PT_PROFILE_TRAVERSAL_COUNTS));
+    h_ctr_->tail_limit = tail_limit(tuning_.tail_paths, p.group_tail > 0, single && single->num_nodes < kSmallTree, busy.others);
+    PTW_CUDA(cudaMemcpyAsync(ctr_.ptr, h_ctr_, sizeof(Counters), cudaMemcpyHostToDevice, stream_));
     // A render too small for any iteration to reach the sorting threshold launches no sort kernels.
     if (std::min<uint64_t>(total_work, uint64_t(tuning_.path_capacity)) < kSortMinPaths) {
         p.sort_bits = 0;
@@ -287,10 +291,10 @@ void WavefrontEngine::begin(const DevScene* scenes, const DevView* views, int n_
     ensure_shape();
     std::memset(h_ctr_, 0, sizeof(Counters));
     h_ctr_->parity = 1;
-    h_ctr_->tail_limit = tail_limit(tuning_.tail_paths, false);  // a server shares the GPU between requests
+    cont_params_ = params(scenes, -1, nullptr, views, n_views, false);
+    h_ctr_->tail_limit = tail_limit(tuning_.tail_paths, cont_params_.group_tail > 0, false, 1);  // a server shares the GPU between requests
     tail_limit_ = h_ctr_->tail_limit;
     PTW_CUDA(cudaMemcpyAsync(ctr_.ptr, h_ctr_, sizeof(Counters), cudaMemcpyHostToDevice, stream_));
-    cont_params_ = params(scenes, -1, nullptr, views, n_views, false);
 }
 
 void WavefrontEngine::update_scheduling(const Tuning& t) {
@@ -312,6 +316,7 @@ void WavefrontEngine::update_scheduling(const Tuning& t) {
     cont_params_.shadow_refill = fresh.shadow_refill;
     cont_params_.walk_burst = fresh.walk_burst;
     cont_params_.pair_visits = fresh.pair_visits;
+    cont_params_.group_tail = fresh.group_tail;
     if (cont_params_.sort_bits > 0) cont_params_.sort_bits = tuning_.sort_rays;
 }
 

@@ -23,6 +23,16 @@ class SvgfDenoiser;
 constexpr int kTailAuto = -2;
 constexpr int kTailAlone = 1 << 17;
 constexpr int kTailShared = 1 << 16;
+// The same where the tail walks rays by groups of eight lanes (WfParams::group_tail): it takes half the time
+// of a thread per path up to 16,384 paths and loses above, and beside other renders it yields sooner.
+// Terrain of 262K triangles, 57,600 paths alone: 1.12 ms with 131,072, 0.93 with 16,384; 1600x900 real-time
+// frames, frames/s with 131,072 (alone) or 65,536 / 16,384 / 8,192 / 4,096: one session 399 / 436 / 401 /
+// 376, two 599 / 600 / 598 / 580, four 699 / 703 / 766 / 770, eight 706 / 704 / 803 / 851.
+constexpr int kGroupTailAlone = 1 << 14;
+constexpr int kGroupTailFew = 1 << 13;   // one or two other renders; or a tree of fewer than kSmallTree nodes (the
+                                         // 36-triangle box, 16,384 paths: 0.28 ms with 16,384, 0.26 with 8,192)
+constexpr int kSmallTree = 512;
+constexpr int kGroupTailMany = 1 << 12;
 
 // Tunable launch parameters (the autotuner's knobs).
 struct Tuning {
@@ -107,6 +117,7 @@ public:
     void set_order_free(bool all) {
         order_free_ = all;
         cont_params_.order_free = all ? 1 : 0;
+        if (!all) cont_params_.group_tail = 0;
     }
 
     const Counters& last() const { return last_; }

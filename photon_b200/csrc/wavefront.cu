@@ -19,6 +19,7 @@
 #include "gbuffer.cuh"
 
 #include "pt_traverse.cuh"
+#include "group_walk.cuh"
 
 namespace ptw {
 
@@ -1111,7 +1112,10 @@ __global__ void __launch_bounds__(256) k_shade(const __grid_constant__ WfParams 
     }
     __shared__ uint32_t s_base, s_hist[kShadeKeys], s_perm[kMaxShadeWindow], s_kr[kMaxShadeWindow];
     const uint32_t tid = threadIdx.x;
-    const uint32_t rounds = min(uint32_t(P.sort_material) * (c->sorting ? 4u : 1u), kMaxShadeRounds);
+    // (A short queue takes shorter windows, down to one path per thread, so that every block has one: 100,000
+    // paths were shaded by 98 of the 296 blocks, four rounds each, in 85 us.)
+    const uint32_t share = (n + gridDim.x * blockDim.x - 1) / (gridDim.x * blockDim.x);
+    const uint32_t rounds = min(min(uint32_t(P.sort_material) * (c->sorting ? 4u : 1u), kMaxShadeRounds), max(share, 1u));
     const uint32_t window = rounds * blockDim.x;
     for (;;) {
         if (tid == 0) s_base = atomicAdd(&c->fetch[2], window);
@@ -1288,12 +1292,15 @@ __global__ void __launch_bounds__(128, 5) k_shade_ordered(const __grid_constant_
     }
 }
 
-// ---- tail: the last queued paths, each finished by one thread --------------------------------------------
+// ---- tail: the last queued paths, each finished by one thread or a group of eight ---------------------------
 // Once no new paths remain and few are queued, an iteration's kernels have too little work to cover
-// the latency of their longest ray, and every remaining bounce would pay that again. k_tail takes the
-// whole queue instead: each thread traces, shades and shadow-tests its path bounce after bounce, in
-// the order of the queued kernels (emission, then the light sample's contribution, then the next
-// bounce), so each path's result is the same as through the queues.
+// the latency of their longest ray, and every remaining bounce would pay that again. The tail takes the
+// whole queue instead: each path is traced, shaded and shadow-tested bounce after bounce, in the order of
+// the queued kernels (emission, then the light sample's contribution, then the next bounce), so each
+// path's result is the same as through the queues. What bounds it is the longest path: a ray that grazes
+// the 262K scene's height field walks hundreds of nodes, one dependent read after another. So a tail of at
+// most P.group_tail paths goes to k_tail_group, eight lanes per path over an 8-wide tree; a larger one to
+// k_tail, a thread per path.
 template <bool Count, bool Packed>
 __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ WfParams P) {
     Counters* c = P.ctr;
@@ -1301,6 +1308,7 @@ __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ WfParams P
     extern __shared__ int smem_stack[];
     int* stack = smem_stack + threadIdx.x;
     const uint32_t p = c->parity, n = c->count[p];
+    if (n <= P.group_tail) return;  // k_tail_group's
     TraversalCounters tc{0, 0}, ts{0, 0};
     unsigned long long rays = 0, shadow_rays = 0;
     for (;;) {
@@ -1337,6 +1345,73 @@ __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ WfParams P
         warp_add_u64(&c->tri_tests, tc.tris);
         warp_add_u64(&c->shadow_node_visits, ts.nodes);
         warp_add_u64(&c->shadow_tri_tests, ts.tris);
+    }
+}
+
+// A group of eight lanes per path, four paths per warp in lockstep: the groups' rays are walked together
+// (group_walk.cuh) and their vertices shaded together, each lane of a group computing the same. Bound by the
+// longest path up to some 8,000 paths (the groups in flight), then by issue, which is why larger tails go
+// to k_tail. Frames of the 262K terrain, depth 8, a thread per path -> groups: 4,096 paths 0.97 -> 0.36 ms,
+// 14,400 1.03 -> 0.49, 57,600 1.12 -> 1.2 (not taken); the 36-triangle box, whose rays are short: 4,096
+// paths 0.23 -> 0.20, 16,384 0.27 -> 0.28. (Groups that step on their own, each with the warp masks of its
+// own lanes, run one after another: 14,400 paths 0.56. Leaving a thread's path to the groups after 128 to
+// 512 walk steps: 57,600 paths 1.05-1.2 ms, 115,200 1.24-1.6 against 1.17: not kept.)
+__global__ void __launch_bounds__(128) k_tail_group(const __grid_constant__ WfParams P) {
+    Counters* c = P.ctr;
+    if (!c->tail) return;
+    const uint32_t p = c->parity, n = c->count[p];
+    if (n > P.group_tail) return;
+    __shared__ uint2 s_stack[128 / kWide][kGroupStack];
+    uint2* stack = s_stack[threadIdx.x / kWide];
+    const uint32_t gl = threadIdx.x & (kWide - 1);
+    uint32_t rays = 0, shadow_rays = 0;
+    PathState st{};
+    const DevScene* s = P.scenes;
+    bool has = false, first = true, cont = false, drained = false;
+    for (;;) {
+        // Each group without a path claims one.
+        uint32_t k = n;
+        if (!has && !drained && gl == 0) k = atomicAdd(&c->fetch[5], 1u);
+        k = __shfl_sync(kFull, k, 0, kWide);
+        if (!has) {
+            drained = k >= n;
+            if (!drained) {
+                st = load_path(P, p, k);
+                s = &scene_for(P, st.id.x);
+                has = first = true;
+            }
+        }
+        if (!__any_sync(kFull, has)) break;
+        Hit h{kInf, -1, 0.0f, 0.0f};
+        group_walk<false>(has, stack, *s, st.ro, st.rd, kInf, h);
+        bool shadow = false;
+        ShadowRay sh{};
+        if (has) {
+            if (!first) rays++;  // the setup counted each queued path's first ray
+            first = false;
+            cont = shade_vertex(P, st, make_float4(h.t, __int_as_float(h.tri), h.u, h.v), shadow, sh);
+        }
+        __syncwarp();
+        if (__any_sync(kFull, shadow)) {
+            Hit hs{kInf, -1, 0.0f, 0.0f};
+            const bool occluded = group_walk<true>(shadow, stack, *s, sh.o, sh.d, sh.tmax, hs);
+            if (shadow) {
+                shadow_rays++;
+                if (!occluded) st.L = st.L + sh.c;
+            }
+        }
+        if (has && !cont) {
+            if (gl == 0) {
+                const DevView& v = P.views[st.id.x];
+                v.sample_out[st.id.y] = make_float4(st.L.x, st.L.y, st.L.z, 0.0f);
+                if (v.done_counter) atomicAdd(v.done_counter, 1ull);
+            }
+            has = false;
+        }
+    }
+    if (gl == 0) {
+        if (rays) atomicAdd(&c->rays, (unsigned long long)rays);
+        if (shadow_rays) atomicAdd(&c->shadow_rays, (unsigned long long)shadow_rays);
     }
 }
 
@@ -1951,6 +2026,9 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shadow<false, true, true, false>, trace_block, smem);
     if (e != cudaSuccess) return e;
     out->shadow_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tail_group, 128, 0);
+    if (e != cudaSuccess) return e;
+    out->group_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     out->shade_block = shade_block;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade, shade_block, 0);
     if (e != cudaSuccess) return e;
@@ -2010,6 +2088,7 @@ static void launch_tail(const WfParams& p, const LaunchShape& ls, cudaStream_t s
         if (p.packed) k_tail<false, true><<<ls.trace_grid, ls.trace_block, smem, stream>>>(p);
         else k_tail<false, false><<<ls.trace_grid, ls.trace_block, smem, stream>>>(p);
     }
+    if (p.group_tail) k_tail_group<<<ls.group_grid, 128, 0, stream>>>(p);
 }
 
 cudaError_t wf_iteration(const WfParams& p, const LaunchShape& ls, cudaStream_t stream, cudaEvent_t* ev) {

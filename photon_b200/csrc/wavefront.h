@@ -90,6 +90,7 @@ struct WfParams {
     int packed;                // 1: f32x2 slab tests in the traversal kernels
     uint32_t tail_paths;       // > 0: once no new paths remain and at most Counters::tail_limit are queued,
                                // finish them in one kernel (one thread per path, all bounces)
+    uint32_t group_tail;       // a tail of at most this many paths takes eight lanes per path (k_tail_group; 0: none)
     int wide_shadows;          // 1: shadow rays walk the 4-wide BVH where the scene has one
     uint32_t trace_refill;     // 1-32: a trace warp claims new rays once fewer of its lanes hold one
     uint32_t shadow_refill;    // the same for the shadow walk
@@ -129,6 +130,7 @@ struct LaunchShape {
     int pair_trace_grid, pair_shadow_grid;  // the pair walks (more shared memory per block)
     int list_trace_grid, list_shadow_grid;  // the list walks
     int ordered_grid, misses_grid;          // shading in class order
+    int group_grid;                         // the tail by groups of lanes
 };
 
 // Fills grid sizes from the occupancy of each kernel on `device` (block sizes as requested).
@@ -142,9 +144,10 @@ cudaError_t wf_iteration(const WfParams& p, const LaunchShape& ls, cudaStream_t 
 constexpr uint32_t kSortMinPaths = 1u << 21;
 // Renders of fewer paths are not shaded in class order over the whole queue.
 constexpr uint32_t kOrderMinPaths = 1u << 18;
+constexpr uint32_t kGroupTail = 1u << 14;  // WfParams::group_tail where every scene has the 8-wide tree
 // Kernels wf_iteration launches for these parameters.
 inline int wf_kernels_per_iteration(const WfParams& p) {
-    return 5 + (p.order ? 3 : 0) + (p.tail_paths > 0 ? 1 : 0) + (p.sort_bits > 0 ? 3 : 0) + (p.shadow_sort_bits > 0 ? 2 : 0);
+    return 5 + (p.order ? 3 : 0) + (p.tail_paths > 0 ? (p.group_tail ? 2 : 1) : 0) + (p.sort_bits > 0 ? 3 : 0) + (p.shadow_sort_bits > 0 ? 2 : 0);
 }
 // Sums the samples of every pixel of a view in sample order (after a pass).
 cudaError_t wf_accumulate(const DevView* d_view, const DevView& h_view, int first_pass, int last_pass, cudaStream_t stream);
