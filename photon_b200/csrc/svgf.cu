@@ -58,6 +58,16 @@ __device__ __forceinline__ float log_normal_weight(V3 n, float ex, float ey, flo
     float c = fmaxf(0.0f, dot(n, v) * rsqrtf(dot(v, v)));
     return c > 0.0f ? phi * __logf(c) : (phi > 0.0f ? -kInf : 0.0f);
 }
+// The octahedral direction with the scale that normalises it: what log_normal_weight takes from a record.
+// A tile's kernels prepare it once per staged pixel instead of once per tap (25 or 49 of them).
+__device__ __forceinline__ float4 tap_direction(float ex, float ey) {
+    V3 v = oct_direction(ex, ey);
+    return make_float4(v.x, v.y, v.z, rsqrtf(dot(v, v)));
+}
+__device__ __forceinline__ float log_normal_weight(V3 n, float4 dir, float phi) {
+    float c = fmaxf(0.0f, dot(n, xyz(dir)) * dir.w);
+    return c > 0.0f ? phi * __logf(c) : (phi > 0.0f ? -kInf : 0.0f);
+}
 __device__ __forceinline__ int edge_material(float4 e) { return __float_as_int(e.w); }
 
 __device__ __forceinline__ V3 demodulate(V3 color, V3 emission, V3 albedo) {
@@ -155,46 +165,93 @@ __global__ void __launch_bounds__(128) k_temporal(Frame5 in5, SvgfFrame in, Prev
 
 // variance_kernel (svgf.cu:96-132): from the moments, or a 7x7 bilateral estimate while the
 // history is shorter than 4 frames. The edge-stopping weights use the fast exp / pow that Photon's
-// build (--use_fast_math) gives svgf.cu.
-__global__ void __launch_bounds__(128) k_variance(const float4* __restrict__ edge, int w, int h, const float4* __restrict__ illum,
-                                                  const float4* __restrict__ moments, float phi_normal, float4* __restrict__ out) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    int i = y * w + x;
-    float4 cc = __ldg(illum + i);
-    V3 c = xyz(cc);
-    float len = cc.w;
-    float variance = __ldg(moments + i).z;
-    float4 e = __ldg(edge + i);
-    int mat = edge_material(e);
-    if (len < 4.0f && mat >= 0) {
-        V3 n = oct_decode(e.x, e.y);
-        float z = e.z;
-        float inv_dz = __fdividef(1.0f, 0.05f * z + 1e-3f);
-        float wsum = 0, m1 = 0, m2 = 0;
-        V3 acc = v3(0);
-        for (int dy = -3; dy <= 3; dy++)
-            for (int dx = -3; dx <= 3; dx++) {
-                int xx = x + dx, yy = y + dy;
-                if (xx < 0 || yy < 0 || xx >= w || yy >= h) continue;
-                int j = yy * w + xx;
-                float4 ej = __ldg(edge + j);
-                if (edge_material(ej) != mat) continue;
-                float wt = __expf(log_normal_weight(n, ej.x, ej.y, phi_normal) - fabsf(ej.z - z) * inv_dz);
-                float4 m = __ldg(moments + j);
-                m1 += m.x * wt;
-                m2 += m.y * wt;
-                acc = acc + xyz(__ldg(illum + j)) * wt;
-                wsum += wt;
-            }
-        if (wsum > 0) {
-            m1 /= wsum;
-            m2 /= wsum;
-            variance = fmaxf(0.0f, m2 - m1 * m1) * (4.0f / len);
-            c = acc / wsum;
+// build (--use_fast_math) gives svgf.cu. A block whose pixels need the estimate stages its pixels and a
+// border of three in shared memory with their directions prepared, once per staged pixel instead of once
+// per tap. With two pixels per thread (Px), one above the other, whose windows share six of eight rows, fewer
+// shared-memory reads bound it (85% of their peak with one). 1600x900, every pixel a surface: 155 us (global
+// loads, directions per tap) -> 98 (staged) -> 83 (two pixels); 427x241, whose 224 blocks of two-pixel threads
+// do not fill the chip: 22.6 -> 13.6 with one, 17.1 with two. So frames below kVarPairs pixels take one.
+constexpr int kVarW = 32, kVarRows = 8, kVarR = 3;  // a block's threads, the window's radius
+constexpr int kVarPairs = 400000;
+template <int Px>
+__global__ void __launch_bounds__(kVarW* kVarRows) k_variance(const float4* __restrict__ edge, int w, int h, const float4* __restrict__ illum,
+                                                               const float4* __restrict__ moments, float phi_normal,
+                                                               float4* __restrict__ out) {
+    constexpr int kVarH = kVarRows * Px, kTw = kVarW + 2 * kVarR, kTh = kVarH + 2 * kVarR;
+    __shared__ float4 t_dir[kTh * kTw], t_zm[kTh * kTw], t_col[kTh * kTw];  // direction; depth, material, moments; colour
+    const int tx = threadIdx.x, ty = Px * int(threadIdx.y), x = blockIdx.x * kVarW + tx, y = blockIdx.y * kVarH + ty;
+    V3 c[Px], n[Px];
+    float variance[Px], len[Px], z[Px], inv_dz[Px];
+    int mat[Px];
+    bool estimate[Px], some = false;
+#pragma unroll
+    for (int k = 0; k < Px; k++) {
+        const bool on = x < w && y + k < h;
+        float4 cc = make_float4(0, 0, 0, 0), e = cc;
+        variance[k] = 0;
+        if (on) {
+            const int i = (y + k) * w + x;
+            cc = __ldg(illum + i);
+            variance[k] = __ldg(moments + i).z;
+            e = __ldg(edge + i);
         }
+        c[k] = xyz(cc);
+        len[k] = cc.w;
+        mat[k] = edge_material(e);
+        estimate[k] = on && len[k] < 4.0f && mat[k] >= 0;
+        some = some || estimate[k];
+        n[k] = oct_decode(e.x, e.y);
+        z[k] = e.z;
+        inv_dz[k] = __fdividef(1.0f, 0.05f * e.z + 1e-3f);
     }
-    out[i] = make_float4(c.x, c.y, c.z, variance);
+    if (__syncthreads_or(some)) {
+        for (int k = int(threadIdx.y) * kVarW + tx; k < kTw * kTh; k += kVarW * kVarRows) {
+            const int xx = int(blockIdx.x) * kVarW + k % kTw - kVarR, yy = int(blockIdx.y) * kVarH + k / kTw - kVarR;
+            float4 dir = make_float4(0, 0, 0, 0), zm = make_float4(0, __int_as_float(-1), 0, 0), col = dir;  // (no pixel: no surface)
+            if (xx >= 0 && yy >= 0 && xx < w && yy < h) {
+                const int j = yy * w + xx;
+                const float4 ej = __ldg(edge + j), m = __ldg(moments + j);
+                dir = tap_direction(ej.x, ej.y);
+                zm = make_float4(ej.z, ej.w, m.x, m.y);
+                col = __ldg(illum + j);
+            }
+            t_dir[k] = dir;
+            t_zm[k] = zm;
+            t_col[k] = col;
+        }
+        __syncthreads();
+    }
+    if (some) {
+        float wsum[Px] = {}, m1[Px] = {}, m2[Px] = {};
+        V3 acc[Px] = {};
+        for (int dy = -kVarR; dy < kVarR + Px; dy++)
+#pragma unroll
+            for (int dx = -kVarR; dx <= kVarR; dx++) {
+                const int j = (ty + kVarR + dy) * kTw + tx + kVarR + dx;
+                const float4 zm = t_zm[j], dir = t_dir[j], col = t_col[j];
+                const int m = __float_as_int(zm.y);
+#pragma unroll
+                for (int k = 0; k < Px; k++) {
+                    if (m != mat[k] || dy < k - kVarR || dy > k + kVarR) continue;
+                    float wt = __expf(log_normal_weight(n[k], dir, phi_normal) - fabsf(zm.x - z[k]) * inv_dz[k]);
+                    m1[k] += zm.z * wt;
+                    m2[k] += zm.w * wt;
+                    acc[k] = acc[k] + xyz(col) * wt;
+                    wsum[k] += wt;
+                }
+            }
+#pragma unroll
+        for (int k = 0; k < Px; k++)
+            if (estimate[k] && wsum[k] > 0) {
+                m1[k] /= wsum[k];
+                m2[k] /= wsum[k];
+                variance[k] = fmaxf(0.0f, m2[k] - m1[k] * m1[k]) * (4.0f / len[k]);
+                c[k] = acc[k] / wsum[k];
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < Px; k++)
+        if (x < w && y + k < h) out[(y + k) * w + x] = make_float4(c[k].x, c[k].y, c[k].z, variance[k]);
 }
 
 struct AtrousEpilogue {
@@ -289,6 +346,122 @@ __global__ void __launch_bounds__(128) k_atrous(const float4* __restrict__ edge,
     if (ep.output) ep.output[i] = remodulate(ep, i, mat, result);
 }
 
+// ---- a-trous passes over staged tiles ------------------------------------------------------------------------
+// A tile's pixel, staged once and read by up to 25 taps: the filtered colour and variance; the colour's
+// luminance, (unused), depth and material; the normal's direction (tap_direction). A place outside the image
+// has material -2, which no surface has, so a tap needs no test of its coordinates.
+struct AtrousTile {
+    float4 *src, *edge, *dir;
+    __device__ __forceinline__ void prepare(int k, float4 s, float4 e, bool inside) {
+        dir[k] = tap_direction(e.x, e.y);
+        edge[k] = make_float4(luminance(xyz(s)), 0.0f, e.z, inside ? e.w : __int_as_float(-2));
+    }
+};
+
+// Preparing a record once per staged pixel takes the direction, its reciprocal root and the luminance, 25 of a
+// tap's 70 instructions, out of the 25 taps; the passes are bound by issue (79%). 1600x900, every pixel a
+// surface, per pass of steps 1 / 2 / 4 / 8 / 16: 94 / 89 / 89 / 100 / 101 us -> 73 / 68 / 76 / 73 / 91 (85 /
+// 79 / 83 / 81 / 98 before denormals were flushed). Strided TMA tiles for steps 8 and 16 took 127 and 154.
+//
+// atrous_kernel's filter (svgf.cu:134-186) at pixel (x, y), entry ci of the tile, whose taps lie sx and sy
+// entries apart in x and y. The 3x3 variances and the depth gradient come through src_w(x, y) and
+// depth(x, y), called with coordinates inside the image.
+template <typename SrcW, typename Depth>
+__device__ __forceinline__ float4 atrous_filter(const AtrousTile& t, int ci, int sx, int sy, int x, int y, int w, int h, int step, float4 center,
+                                                float4 ec, float phi_color, float phi_normal, float phi_depth, SrcW src_w, Depth depth) {
+    const int mat = edge_material(ec);
+    if (mat < 0) return center;
+    float var = 0, vw = 0;
+#pragma unroll
+    for (int dy = -1; dy <= 1; dy++)
+#pragma unroll
+        for (int dx = -1; dx <= 1; dx++) {
+            int xx = min(max(x + dx, 0), w - 1), yy = min(max(y + dy, 0), h - 1);
+            float k = (dx == 0 && dy == 0) ? 0.25f : ((dx == 0 || dy == 0) ? 0.125f : 0.0625f);
+            var += src_w(xx, yy) * k;
+            vw += k;
+        }
+    var /= vw;
+    V3 nrm = oct_decode(ec.x, ec.y);
+    float z = ec.z;
+    float zx = depth(min(x + 1, w - 1), y) - depth(max(x - 1, 0), y);
+    float zy = depth(x, min(y + 1, h - 1)) - depth(x, max(y - 1, 0));
+    float grad = 0.5f * fmaxf(fabsf(zx), fabsf(zy));
+    float lum_c = luminance(xyz(center));
+    float sigma_l = phi_color * sqrtf(fmaxf(var, 0.0f)) + 1e-4f;
+    float inv_sigma = __fdividef(1.0f, sigma_l);
+    const float gs = phi_depth * grad * float(step), dz0 = 1e-3f * z + 1e-4f;
+    const float inv_dz[6] = {__fdividef(1.0f, dz0), __fdividef(1.0f, gs + dz0), __fdividef(1.0f, gs * 1.41421356f + dz0),
+                             __fdividef(1.0f, gs * 2.0f + dz0), __fdividef(1.0f, gs * 2.23606798f + dz0),
+                             __fdividef(1.0f, gs * 2.82842712f + dz0)};
+    const float kernel[3] = {3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
+    V3 sum = v3(0);
+    float wsum = 0, vsum = 0;
+#pragma unroll
+    for (int dy = -2; dy <= 2; dy++)
+#pragma unroll
+        for (int dx = -2; dx <= 2; dx++) {
+            const int tj = ci + dy * sy + dx * sx;
+            const float4 ej = t.edge[tj];
+            if (edge_material(ej) != mat) continue;
+            const float4 sj = t.src[tj];
+            const int r2 = dx * dx + dy * dy;
+            const int di = r2 == 0 ? 0 : r2 == 1 ? 1 : r2 == 2 ? 2 : r2 == 4 ? 3 : r2 == 5 ? 4 : 5;
+            float k = kernel[abs(dx)] * kernel[abs(dy)];
+            float arg = log_normal_weight(nrm, t.dir[tj], phi_normal) - fabsf(ej.x - lum_c) * inv_sigma - fabsf(ej.z - z) * inv_dz[di];
+            float wt = k * __expf(arg);
+            sum = sum + xyz(sj) * wt;
+            vsum += wt * wt * sj.w;
+            wsum += wt;
+        }
+    if (!(wsum > 0)) return center;
+    V3 rr = sum / wsum;
+    return make_float4(rr.x, rr.y, rr.z, vsum / (wsum * wsum));
+}
+
+__device__ __forceinline__ void atrous_write(const AtrousEpilogue& ep, float4* dst, int i, float4 result, float4 ec) {
+    dst[i] = result;
+    if (ep.prev_illum) {
+        ep.prev_illum[i] = make_float4(result.x, result.y, result.z, __ldg(ep.illum + i).w);
+        ep.prev_moments[i] = __ldg(ep.moments + i);
+        ep.prev_edge[i] = ec;
+    }
+    if (ep.output) ep.output[i] = remodulate(ep, i, edge_material(ec), result);
+}
+
+// A pass of a large step: a block's 32 x 8 outputs are rows `step` apart, so that its taps fall into 12 rows
+// of 32 + 4 step pixels, which it loads whole (coalesced) and prepares. Against global loads per tap, whose
+// 25 x 32 bytes per pixel came mostly from L2, each byte is read 3 to 5 times instead of 25.
+constexpr int kRowsW = 32, kRowsH = 8;
+__host__ __device__ constexpr int rows_tile(int step) { return (kRowsH + 4) * (kRowsW + 4 * step); }
+size_t rows_smem_bytes(int step) { return 3 * sizeof(float4) * size_t(rows_tile(step)); }
+__global__ void __launch_bounds__(kRowsW* kRowsH) k_atrous_rows(const float4* __restrict__ edge, int w, int h, int step, float phi_color,
+                                                                float phi_normal, float phi_depth, const float4* __restrict__ src,
+                                                                float4* __restrict__ dst, AtrousEpilogue ep) {
+    extern __shared__ __align__(128) float4 tile_smem[];
+    const int n = rows_tile(step), row = kRowsW + 4 * step;
+    AtrousTile t{tile_smem, tile_smem + n, tile_smem + 2 * n};
+    const int tx = int(threadIdx.x), ty = int(threadIdx.y);
+    const int x0 = int(blockIdx.x) * kRowsW, y0 = int(blockIdx.y) / step * (step * kRowsH) + int(blockIdx.y) % step;
+    for (int k = ty * kRowsW + tx; k < n; k += kRowsW * kRowsH) {
+        const int xx = x0 + k % row - 2 * step, yy = y0 + (k / row - 2) * step;
+        const bool inside = xx >= 0 && yy >= 0 && xx < w && yy < h;
+        const int j = inside ? yy * w + xx : 0;
+        const float4 s = __ldg(src + j), e = __ldg(edge + j);
+        t.src[k] = s;
+        t.prepare(k, s, e, inside);
+    }
+    __syncthreads();
+    const int x = x0 + tx, y = y0 + ty * step;
+    if (x >= w || y >= h) return;
+    const int i = y * w + x, ci = (ty + 2) * row + tx + 2 * step;
+    const float4 ec = __ldg(edge + i);
+    const float4 result = atrous_filter(t, ci, step, row, x, y, w, h, step, t.src[ci], ec, phi_color, phi_normal, phi_depth,
+                                        [&](int xx, int yy) { return __ldg(src + yy * w + xx).w; },
+                                        [&](int xx, int yy) { return __ldg(edge + yy * w + xx).z; });
+    atrous_write(ep, dst, i, result, ec);
+}
+
 // ---- a-trous passes with TMA-staged tiles ------------------------------------------------------------------
 // A pass with step s reads, for each pixel, the 5 x 5 taps at offsets (dx, dy) * s. A block takes a
 // 16 x 16 tile of pixels on a grid of spacing e (e = 1: a contiguous tile) whose taps lie r = s / e
@@ -305,7 +478,7 @@ constexpr unsigned long long kTmaDrainNs = 2000000000ull;  // after a timeout: t
 constexpr unsigned long long kTmaTestWaitNs = 2000ull;     // the test mode's waits (no copy is issued)
 
 __host__ __device__ constexpr int tma_box_side(int r) { return kTmaTile + 4 * r; }
-size_t tma_smem_bytes(int r) { return 2 * size_t(tma_box_side(r)) * size_t(tma_box_side(r)) * sizeof(float4) + 16; }
+size_t tma_smem_bytes(int r) { return 3 * size_t(tma_box_side(r)) * size_t(tma_box_side(r)) * sizeof(float4) + 16; }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
@@ -344,7 +517,8 @@ __global__ void __launch_bounds__(kTmaTile * kTmaTile) k_atrous_tma(const __grid
     const int n = tma_box_side(r);  // box side in grid cells
     float4* t_src = tile_smem;
     float4* t_edge = tile_smem + n * n;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(tile_smem + 2 * n * n);
+    float4* t_dir = tile_smem + 2 * n * n;  // the taps' directions, prepared below
+    uint64_t* bar = reinterpret_cast<uint64_t*>(tile_smem + 3 * n * n);
     const int rx = int(blockIdx.z) % e, ry = int(blockIdx.z) / e;
     const int cx0 = int(blockIdx.x) * kTmaTile, cy0 = int(blockIdx.y) * kTmaTile;
     const bool leader = threadIdx.x == 0 && threadIdx.y == 0;
@@ -398,72 +572,25 @@ __global__ void __launch_bounds__(kTmaTile * kTmaTile) k_atrous_tma(const __grid
     }
     const int tx = int(threadIdx.x), ty = int(threadIdx.y);
     const int x = rx + e * (cx0 + tx), y = ry + e * (cy0 + ty);
-    if (x >= w || y >= h) return;
     const int i = y * w + x, step = e * r;
     const int ci = (ty + 2 * r) * n + (tx + 2 * r);
-    float4 center = t_src[ci];
-    float4 ec = t_edge[ci];
-    int mat = edge_material(ec);
-    float4 result = center;
-    if (mat >= 0) {
-        float var = 0, vw = 0;
-#pragma unroll
-        for (int dy = -1; dy <= 1; dy++)
-#pragma unroll
-            for (int dx = -1; dx <= 1; dx++) {
-                int xx = min(max(x + dx, 0), w - 1), yy = min(max(y + dy, 0), h - 1);
-                float k = (dx == 0 && dy == 0) ? 0.25f : ((dx == 0 || dy == 0) ? 0.125f : 0.0625f);
-                var += __ldg(src + yy * w + xx).w * k;
-                vw += k;
-            }
-        var /= vw;
-        V3 nrm = oct_decode(ec.x, ec.y);
-        float z = ec.z;
-        float zx = __ldg(edge + y * w + min(x + 1, w - 1)).z - __ldg(edge + y * w + max(x - 1, 0)).z;
-        float zy = __ldg(edge + min(y + 1, h - 1) * w + x).z - __ldg(edge + max(y - 1, 0) * w + x).z;
-        float grad = 0.5f * fmaxf(fabsf(zx), fabsf(zy));
-        float lum_c = luminance(xyz(center));
-        float sigma_l = phi_color * sqrtf(fmaxf(var, 0.0f)) + 1e-4f;
-        float inv_sigma = __fdividef(1.0f, sigma_l);
-        const float gs = phi_depth * grad * float(step), dz0 = 1e-3f * z + 1e-4f;
-        const float inv_dz[6] = {__fdividef(1.0f, dz0), __fdividef(1.0f, gs + dz0), __fdividef(1.0f, gs * 1.41421356f + dz0),
-                                 __fdividef(1.0f, gs * 2.0f + dz0), __fdividef(1.0f, gs * 2.23606798f + dz0),
-                                 __fdividef(1.0f, gs * 2.82842712f + dz0)};
-        const float kernel[3] = {3.0f / 8.0f, 1.0f / 4.0f, 1.0f / 16.0f};
-        V3 sum = v3(0);
-        float wsum = 0, vsum = 0;
-#pragma unroll
-        for (int dy = -2; dy <= 2; dy++)
-#pragma unroll
-            for (int dx = -2; dx <= 2; dx++) {
-                int xx = x + dx * step, yy = y + dy * step;
-                if (xx < 0 || yy < 0 || xx >= w || yy >= h) continue;
-                int tj = ci + dy * r * n + dx * r;
-                float4 ej = t_edge[tj];
-                if (edge_material(ej) != mat) continue;
-                float4 sj = t_src[tj];
-                const int r2 = dx * dx + dy * dy;
-                const int di = r2 == 0 ? 0 : r2 == 1 ? 1 : r2 == 2 ? 2 : r2 == 4 ? 3 : r2 == 5 ? 4 : 5;
-                float k = kernel[abs(dx)] * kernel[abs(dy)];
-                float arg = log_normal_weight(nrm, ej.x, ej.y, phi_normal) - fabsf(luminance(xyz(sj)) - lum_c) * inv_sigma -
-                            fabsf(ej.z - z) * inv_dz[di];
-                float wt = k * __expf(arg);
-                sum = sum + xyz(sj) * wt;
-                vsum += wt * wt * sj.w;
-                wsum += wt;
-            }
-        if (wsum > 0) {
-            V3 rr = sum / wsum;
-            result = make_float4(rr.x, rr.y, rr.z, vsum / (wsum * wsum));
-        }
+    const float4 center = t_src[ci];
+    const float4 ec = t_edge[ci];
+    __syncthreads();
+    // What every tap would compute from its record, once per staged pixel.
+    AtrousTile t{t_src, t_edge, t_dir};
+    for (int k = ty * kTmaTile + tx; k < n * n; k += kTmaTile * kTmaTile) {
+        const int xx = rx + e * (cx0 + k % n - 2 * r), yy = ry + e * (cy0 + k / n - 2 * r);
+        t.prepare(k, t_src[k], t_edge[k], xx >= 0 && yy >= 0 && xx < w && yy < h);
     }
-    dst[i] = result;
-    if (ep.prev_illum) {
-        ep.prev_illum[i] = make_float4(result.x, result.y, result.z, __ldg(ep.illum + i).w);
-        ep.prev_moments[i] = __ldg(ep.moments + i);
-        ep.prev_edge[i] = ec;
-    }
-    if (ep.output) ep.output[i] = remodulate(ep, i, mat, result);
+    __syncthreads();
+    if (x >= w || y >= h) return;
+    // (A contiguous tile holds the pixel's neighbours too.)
+    const int origin = Rank == 2 ? (2 * r - cy0) * n + 2 * r - cx0 : 0;
+    const float4 result = atrous_filter(t, ci, r, r * n, x, y, w, h, step, center, ec, phi_color, phi_normal, phi_depth,
+                                        [&](int xx, int yy) { return Rank == 2 ? t_src[origin + yy * n + xx].w : __ldg(src + yy * w + xx).w; },
+                                        [&](int xx, int yy) { return Rank == 2 ? t_edge[origin + yy * n + xx].z : __ldg(edge + yy * w + xx).z; });
+    atrous_write(ep, dst, i, result, ec);
 }
 
 // History and/or remodulation without any a-trous pass (atrous_iterations == 0).
@@ -500,7 +627,10 @@ void denoise(const Frame5& in5, const SvgfFrame& in, const PrevCamera& pc, int w
     const float4* edge = edge_out;
     k_temporal<FromPhoton><<<grid, block, 0, stream>>>(in5, in, pc, w, h, has_history ? 1 : 0, s.alpha_color, s.alpha_moments, hist,
                                                        edge_out, illum, moments);
-    k_variance<<<grid, block, 0, stream>>>(edge, w, h, illum, moments, s.phi_normal, f0);
+    const int px = w * h >= kVarPairs ? 2 : 1, var_rows = kVarRows * px;
+    const dim3 var_grid((w + kVarW - 1) / kVarW, (h + var_rows - 1) / var_rows), var_block(kVarW, kVarRows);
+    if (px == 2) k_variance<2><<<var_grid, var_block, 0, stream>>>(edge, w, h, illum, moments, s.phi_normal, f0);
+    else k_variance<1><<<var_grid, var_block, 0, stream>>>(edge, w, h, illum, moments, s.phi_normal, f0);
     AtrousEpilogue last{};
     last.output = reinterpret_cast<float4*>(output);
     last.color = FromPhoton ? in5.color : in.color;
@@ -531,6 +661,10 @@ void denoise(const Frame5& in5, const SvgfFrame& in, const PrevCamera& pc, int w
                 k_atrous_tma<5><<<tgrid, dim3(kTmaTile, kTmaTile), tma_smem_bytes(tp.r), stream>>>(
                     ms, me, bufs[src], edge, w, h, tp.e, tp.r, s.phi_color, s.phi_normal, s.phi_depth, bufs[1 - src], ep, tma.status,
                     tma.test_no_copy);
+        } else if (tma.passes && it < kTmaPasses && tma.passes[it].e == kRowsPass) {
+            const int step = 1 << it, bands = (h + step * kRowsH - 1) / (step * kRowsH);
+            k_atrous_rows<<<dim3((w + kRowsW - 1) / kRowsW, bands * step), dim3(kRowsW, kRowsH), rows_smem_bytes(step),
+                            stream>>>(edge, w, h, step, s.phi_color, s.phi_normal, s.phi_depth, bufs[src], bufs[1 - src], ep);
         } else {
             k_atrous<<<grid, block, 0, stream>>>(edge, w, h, 1 << it, s.phi_color, s.phi_normal, s.phi_depth, bufs[src], bufs[1 - src],
                                                  ep);
@@ -612,16 +746,21 @@ void SvgfDenoiser::resize(int w, int h) {
 }
 
 // The staging of each a-trous pass for a TMA mode (pt_svgf_set_tma):
+//   0: global loads for all;
 //   1: contiguous tiles for steps 1-8, global loads from step 16 on;
 //   2: contiguous tiles for steps 1-8, a strided tile for step 16;
-//   3: strided tiles (x, y mod min(step, 8)) for steps 1-16.
+//   3: strided tiles (x, y mod min(step, 8)) for steps 1-16;
+//   kTmaDefault: contiguous tiles for steps 1-4 and staged rows (k_atrous_rows) for steps 8 and 16, whose
+//   contiguous tiles would be 48 x 48 and 80 x 80 pixels for 16 x 16 outputs.
 static void tma_passes_for_mode(int mode, TmaPass* out) {
     for (int it = 0; it < kTmaPasses; it++) {
         const int step = 1 << it;
-        if (mode == 3 || (mode == 2 && step == 16)) {
+        if (mode == kTmaDefault && step >= 8) {
+            out[it] = TmaPass{0, kRowsPass, step};
+        } else if (mode == 3 || (mode == 2 && step == 16)) {
             const int e = step < 8 ? step : 8;
             out[it] = TmaPass{5, e, step / e};
-        } else if ((mode == 1 || mode == 2) && step <= 8) {
+        } else if ((mode == 1 || mode == 2 || mode == kTmaDefault) && step <= 8) {
             out[it] = TmaPass{2, 1, step};
         } else {
             out[it] = TmaPass{0, 1, step};
@@ -629,28 +768,31 @@ static void tma_passes_for_mode(int mode, TmaPass* out) {
     }
 }
 
+// The tile kernels' shared memory (up to 3 x 48 x 48 float4). Kernel attributes belong to a device: set once
+// on each device that runs the passes.
+static void allow_tiles() {
+    static std::mutex mu;
+    static std::vector<int> done;
+    int dev = 0;
+    PTW_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(mu);
+    if (size_t(dev) >= done.size()) done.resize(size_t(dev) + 1, 0);
+    if (done[size_t(dev)]) return;
+    const auto most = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    PTW_CUDA(cudaFuncSetAttribute(k_atrous_tma<2>, most, int(tma_smem_bytes(8))));
+    PTW_CUDA(cudaFuncSetAttribute(k_atrous_tma<5>, most, int(tma_smem_bytes(8))));
+    PTW_CUDA(cudaFuncSetAttribute(k_atrous_rows, most, int(rows_smem_bytes(1 << (kTmaPasses - 1)))));
+    done[size_t(dev)] = 1;
+}
+
 void SvgfDenoiser::build_tma_plan() {
     maps_.assign(3 * kTmaPasses, CUtensorMap{});
     maps_ok_ = false;
     tma_passes_for_mode(tma_mode_, passes_);
     if (tma_mode_ == 0 || w_ == 0) return;
+    allow_tiles();
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) return;
-    {
-        // Kernel attributes belong to a device: set them once on each device that runs the passes.
-        // Up to 2 x 48 x 48 float4 of tiles (contiguous, step 8) per block.
-        static std::mutex attr_mu;
-        static std::vector<int> attr_done;
-        int dev = 0;
-        PTW_CUDA(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> g(attr_mu);
-        if (size_t(dev) >= attr_done.size()) attr_done.resize(size_t(dev) + 1, 0);
-        if (!attr_done[size_t(dev)]) {
-            PTW_CUDA(cudaFuncSetAttribute(k_atrous_tma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tma_smem_bytes(8))));
-            PTW_CUDA(cudaFuncSetAttribute(k_atrous_tma<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tma_smem_bytes(8))));
-            attr_done[size_t(dev)] = 1;
-        }
-    }
     float4* bufs[3] = {edge_.ptr, filter_[0].ptr, filter_[1].ptr};
     const int w = w_, h = h_;
     for (int b = 0; b < 3; b++)
@@ -780,8 +922,12 @@ void svgf_run_noalloc(int device, int w, int h, const float* color, const float*
                    reinterpret_cast<const float4*>(pos), reinterpret_cast<const float4*>(emission)};
         // Without history the temporal step reads nothing from earlier calls, and every scratch
         // element a kernel reads was written earlier in this call: nothing needs clearing.
+        // Every staged pass by rows: no tensor map covers the caller's frame in the static scratch.
+        allow_tiles();
+        TmaPass rows[kTmaPasses];
+        for (int it = 0; it < kTmaPasses; it++) rows[it] = TmaPass{0, kRowsPass, 1 << it};
         denoise<true>(in5, SvgfFrame{}, PrevCamera{}, w, h, false, History{}, edge, AtrousEpilogue{}, illum, moments, f0, f1, s, output,
-                      TmaPlan{nullptr, nullptr, nullptr, 0}, stream);
+                      TmaPlan{nullptr, rows, nullptr, 0}, stream);
     } catch (...) {
         cudaSetDevice(previous);
         throw;

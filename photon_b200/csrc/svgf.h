@@ -12,10 +12,14 @@
 namespace ptw {
 
 // How one a-trous pass stages its taps: rank 0 = global loads, 2 = a contiguous TMA tile, 5 = a
-// strided TMA tile (one residue class of x, y mod e); r = step / e grid cells between taps.
+// strided TMA tile (one residue class of x, y mod e); r = step / e grid cells between taps. Rank 0 with
+// e = kRowsPass: rows staged by plain loads (k_atrous_rows).
 struct TmaPass {
     int rank, e, r;
 };
+constexpr int kRowsPass = 0;
+
+constexpr int kTmaDefault = 4;  // the staging used unless set_tma chooses one of 0 to 3
 
 class SvgfDenoiser {
 public:
@@ -56,7 +60,7 @@ private:
     cudaStream_t stream_;
     int w_ = 0, h_ = 0;
     bool has_history_ = false;
-    int tma_mode_ = 1;
+    int tma_mode_ = kTmaDefault;
     bool tma_test_ = false;
     bool maps_ok_ = false;
     std::vector<CUtensorMap> maps_;    // [edge, filter 0, filter 1][pass]
