@@ -484,6 +484,11 @@ __device__ __forceinline__ void walk_queue_pairs4(uint32_t n, uint32_t* claim, u
 constexpr uint32_t kListCap = 128;  // entries of a warp's ring; a round of visits appends up to 64
 constexpr int kListStack = 12;      // stack entries per thread kept in shared memory (16: trace +0.5%)
 constexpr uint32_t kListVisits = 2; // rounds per step, per node visit of a pair walk's step (see walk_queue_list)
+// The least rays that a warp claims of a queue with fewer than 32 for each warp of the grid: half-filled warps
+// issue more, but a lane meets fewer test rounds of the others' leaves and every scheduler has its warps.
+// Frames of the 262K terrain, depth 8, 32 rays to a warp against this: 57,600 paths 0.933 -> 0.842 ms, 115,200
+// 1.19 -> 1.06, 230,400 1.46 -> 1.36, 1.44M 3.21 -> 3.14 (with 4 or 12 within 1% of that).
+constexpr uint32_t kListShare = 8;
 constexpr float kPrune = 1.0f + 1.0f / 1024.0f;
 constexpr float kNearTie = 1.0f + 1.0f / 16384.0f;
 
@@ -615,14 +620,16 @@ __device__ __forceinline__ void walk_queue_list(uint32_t n, uint32_t* claim, uin
     for (;;) {
         uint32_t act = __ballot_sync(kFull, live);
         if (!drained && uint32_t(__popc(act)) < refill) {
-            const uint32_t idle = ~act, want = uint32_t(__popc(idle));
+            // A short queue is spread over all warps, at least kListShare rays to each.
+            const uint32_t idle = ~act, have = uint32_t(__popc(act)), per = max(n / (gridDim.x * (blockDim.x >> 5)) + 1u, kListShare);
+            const uint32_t want = have < per ? min(32u, per) - have : 0u;
             uint32_t base = 0;
             if (lane == 0) base = atomicAdd(claim, want);
             base = __shfl_sync(kFull, base, 0);
             drained = base + want >= n;
             if (!live) {
-                const uint32_t r = base + uint32_t(__popc(idle & below));
-                if (r < n) {
+                const uint32_t k = uint32_t(__popc(idle & below)), r = base + k;
+                if (k < want && r < n) {
                     V3 o, d;
                     const DevScene* scene = nullptr;
                     idx = begin(r, o, d, limit, nodes, scene);
