@@ -79,13 +79,15 @@ void validate_scene(const pt_scene_desc& d, bool lights_only) {
 
 size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
     size_t b = 0;
-    b += size_t(d.num_nodes) * (64 + 96) + size_t(d.num_tris) * (16 * kTriStride + 16);
+    b += size_t(d.num_nodes) * 64 + size_t(d.num_tris) * (16 * kTriStride + 16);
     b += size_t(d.num_vertices) * ((d.normals ? 16 : 0) + (d.uvs ? 8 : 0) + (d.tangents ? 16 : 0));
     b += size_t(d.num_materials) * 80 + size_t(d.num_textures) * 16 + size_t(d.num_texels) * 4 + 1024;
     b += size_t(d.num_emissive) * 24 + size_t(d.num_punctual) * 48;
     if (d.env_texels) b += size_t(d.env_width) * d.env_height * 16 + (size_t(d.env_height) + 1) * 4 + size_t(d.env_height) * (d.env_width + 1) * 4 + size_t(d.env_height) * 4;
     return b + sizeof(DevScene);
 }
+
+size_t DeviceScene::extra_bytes() const { return wide_.bytes() + light_work_.bytes(); }
 
 size_t DeviceScene::device_bytes() const {
     return nodes_.bytes() + nodes4_.bytes() + wide_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
@@ -246,16 +248,24 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.p_punctual = d.p_punctual;
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
     v.bvh_depth = tree_depth_;
-    v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_depth_, s) ? 1 : 0;
-    if (!v.order_free) {
+    try {
+        v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_depth_, s) ? 1 : 0;
+        if (!v.order_free) {
+            wide_.release();
+        } else if (!lights_only || !wide_.ptr) {
+            DeviceBuffer<float4> room;
+            room.allocate(size_t(v.num_nodes) * 2 * kWide);
+            const int n = wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, room.ptr, s);
+            wide_.allocate(size_t(n) * 2 * kWide);
+            PTW_CUDA(cudaMemcpyAsync(wide_.ptr, room.ptr, wide_.bytes(), cudaMemcpyDeviceToDevice, s));
+            PTW_CUDA(cudaStreamSynchronize(s));
+        }
+    } catch (const Error&) {
+        // No memory for the 8-wide tree: the scene is walked in Photon's order, which needs none. (Any other
+        // failure shows again at the synchronisation that ends the upload.)
+        cudaGetLastError();
         wide_.release();
-    } else if (!lights_only || !wide_.ptr) {
-        DeviceBuffer<float4> room;
-        room.allocate(size_t(v.num_nodes) * 2 * kWide);
-        const int n = wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, room.ptr, s);
-        wide_.allocate(size_t(n) * 2 * kWide);
-        PTW_CUDA(cudaMemcpyAsync(wide_.ptr, room.ptr, wide_.bytes(), cudaMemcpyDeviceToDevice, s));
-        PTW_CUDA(cudaStreamSynchronize(s));
+        v.order_free = 0;
     }
     v.wide = wide_.ptr;
     {

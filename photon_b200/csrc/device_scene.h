@@ -81,6 +81,8 @@ public:
     const DevScene* device_view() const { return d_view_.ptr; }
     bool ready() const { return ready_; }
     size_t device_bytes() const;
+    // Of these, what a render can do without (the 8-wide tree, the light rebuild's scratch).
+    size_t extra_bytes() const;
     float extent() const { return extent_; }
     // Bytes a scene will occupy on the device (for admission before upload).
     static size_t estimate_bytes(const pt_scene_desc& d);

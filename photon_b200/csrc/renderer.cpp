@@ -118,9 +118,15 @@ void WavefrontEngine::reserve_paths(uint64_t needed) {
     keys_.allocate(want);
     shadow_keys_.allocate(want);
     shadow_perm_.allocate(want);
-    order_.allocate(want);
-    classes_.allocate(want);
-    class_ctr_.allocate(128);
+    try {
+        order_.allocate(want);
+        classes_.allocate(want);
+        class_ctr_.allocate(128);
+    } catch (const Error&) {  // no memory for the class order: k_shade's windows, which need none
+        cudaGetLastError();
+        order_.release();
+        classes_.release();
+    }
     pb_.capacity = uint32_t(want);
     if (graph_) {
         cudaGraphExecDestroy(graph_);
@@ -139,6 +145,8 @@ void WavefrontEngine::release_paths() {
     classes_.release();
     pb_ = PathBuffers{};
 }
+
+size_t WavefrontEngine::extra_bytes() const { return order_.bytes() + classes_.bytes() + class_ctr_.bytes(); }
 
 size_t WavefrontEngine::device_bytes() const {
     size_t b = ctr_.bytes() + keys_.bytes() + hist_.bytes() + offsets_.bytes() + shadow_keys_.bytes() + shadow_hist_.bytes() +

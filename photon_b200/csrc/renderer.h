@@ -130,6 +130,7 @@ public:
     double kernel_ms[5] = {0, 0, 0, 0, 0};
     uint64_t kernel_launches = 0, iteration_launches = 0;
     size_t device_bytes() const;
+    size_t extra_bytes() const;  // of these, what a render can do without (the shading order)
     int device() const { return device_; }
     cudaStream_t stream() const { return stream_; }
     uint64_t bytes_per_path() const;

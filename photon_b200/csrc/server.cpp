@@ -51,7 +51,9 @@ Server::Server(const pt_server_config& cfg) : cfg_(cfg), device_(cfg.device) {
     created_sort_rays_ = t.sort_rays;
     engine_->set_tuning(t);
     engine_->reserve_paths(uint64_t(t.path_capacity));
-    pool_bytes_ = engine_->device_bytes();
+    // The budget admits by what rendering needs: the extras (5 bytes per path, up to 96 per BVH node; given up
+    // where memory runs out) take no request's place.
+    pool_bytes_ = engine_->device_bytes() - engine_->extra_bytes();
     d_scenes_.allocate(kMaxScenes);
     d_views_.allocate(1024);
     d_done_.allocate(1024);
@@ -89,7 +91,7 @@ Server::Server(const pt_server_config& cfg) : cfg_(cfg), device_(cfg.device) {
         Tuning st;
         st.path_capacity = 1 << 23;  // grown on the first frames to what they need, up to this
         session_engine_->set_tuning(st);
-        lane_idle_bytes_ = session_engine_->device_bytes();
+        lane_idle_bytes_ = session_engine_->device_bytes() - session_engine_->extra_bytes();
     }
     for (Batch& b : batch_) {
         PTW_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&b.ctr), sizeof(Counters), cudaHostAllocDefault));
@@ -173,9 +175,10 @@ int32_t Server::add_scene(const pt_scene_desc& d) {
     // Checked again under the lock that publishes the scene: concurrent add_scene calls all passed the
     // first check before any of them was counted, and the device scene table holds kMaxScenes entries.
     if (int(scenes_.size()) >= kMaxScenes) throw Error{PT_ERR_BUDGET, "too many resident scenes"};
-    if (cfg_.budget_bytes && bytes_in_use_ + pool_bytes_ + scene_bytes_ + scene->device_bytes() > cfg_.budget_bytes)
+    const size_t bytes = scene->device_bytes() - scene->extra_bytes();
+    if (cfg_.budget_bytes && bytes_in_use_ + pool_bytes_ + scene_bytes_ + bytes > cfg_.budget_bytes)
         throw Error{PT_ERR_BUDGET, "the scene does not fit the device-memory budget"};
-    scene_bytes_ += scene->device_bytes();
+    scene_bytes_ += bytes;
     scenes_.push_back(std::move(scene));
     scenes_dirty_ = true;
     st_.scenes = int(scenes_.size());
@@ -575,7 +578,7 @@ void Server::session_loop() {
         }
 
         lk.lock();
-        size_t lane = session_engine_->device_bytes() - lane_idle_bytes_;
+        size_t lane = session_engine_->device_bytes() - session_engine_->extra_bytes() - lane_idle_bytes_;
         pool_bytes_ = pool_bytes_ - lane_bytes_ + lane;
         lane_bytes_ = lane;
         for (Request* r : frames) {
