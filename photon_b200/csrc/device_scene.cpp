@@ -253,12 +253,7 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
         if (!v.order_free) {
             wide_.release();
         } else if (!lights_only || !wide_.ptr) {
-            DeviceBuffer<float4> room;
-            room.allocate(size_t(v.num_nodes) * 2 * kWide);
-            const int n = wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, room.ptr, s);
-            wide_.allocate(size_t(n) * 2 * kWide);
-            PTW_CUDA(cudaMemcpyAsync(wide_.ptr, room.ptr, wide_.bytes(), cudaMemcpyDeviceToDevice, s));
-            PTW_CUDA(cudaStreamSynchronize(s));
+            wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, wide_, s);
         }
     } catch (const Error&) {
         // No memory for the 8-wide tree: the scene is walked in Photon's order, which needs none. (Any other
