@@ -362,6 +362,8 @@ struct AtrousTile {
 // tap's 70 instructions, out of the 25 taps; the passes are bound by issue (79%). 1600x900, every pixel a
 // surface, per pass of steps 1 / 2 / 4 / 8 / 16: 94 / 89 / 89 / 100 / 101 us -> 73 / 68 / 76 / 73 / 91 (85 /
 // 79 / 83 / 81 / 98 before denormals were flushed). Strided TMA tiles for steps 8 and 16 took 127 and 154.
+// A block without a surface prepares and filters nothing: frames of a viewer, half of them sky, 449 -> 458 per
+// second.
 //
 // atrous_kernel's filter (svgf.cu:134-186) at pixel (x, y), entry ci of the tile, whose taps lie sx and sy
 // entries apart in x and y. The 3x3 variances and the depth gradient come through src_w(x, y) and
@@ -443,6 +445,13 @@ __global__ void __launch_bounds__(kRowsW* kRowsH) k_atrous_rows(const float4* __
     AtrousTile t{tile_smem, tile_smem + n, tile_smem + 2 * n};
     const int tx = int(threadIdx.x), ty = int(threadIdx.y);
     const int x0 = int(blockIdx.x) * kRowsW, y0 = int(blockIdx.y) / step * (step * kRowsH) + int(blockIdx.y) % step;
+    const int x = x0 + tx, y = y0 + ty * step, i = y * w + x;
+    const bool on = x < w && y < h;
+    const float4 ec = on ? __ldg(edge + i) : make_float4(0, 0, 0, __int_as_float(-1));
+    if (!__syncthreads_or(edge_material(ec) >= 0)) {  // no surface: nothing to filter, so nothing to stage
+        if (on) atrous_write(ep, dst, i, __ldg(src + i), ec);
+        return;
+    }
     for (int k = ty * kRowsW + tx; k < n; k += kRowsW * kRowsH) {
         const int xx = x0 + k % row - 2 * step, yy = y0 + (k / row - 2) * step;
         const bool inside = xx >= 0 && yy >= 0 && xx < w && yy < h;
@@ -452,10 +461,8 @@ __global__ void __launch_bounds__(kRowsW* kRowsH) k_atrous_rows(const float4* __
         t.prepare(k, s, e, inside);
     }
     __syncthreads();
-    const int x = x0 + tx, y = y0 + ty * step;
-    if (x >= w || y >= h) return;
-    const int i = y * w + x, ci = (ty + 2) * row + tx + 2 * step;
-    const float4 ec = __ldg(edge + i);
+    if (!on) return;
+    const int ci = (ty + 2) * row + tx + 2 * step;
     const float4 result = atrous_filter(t, ci, step, row, x, y, w, h, step, t.src[ci], ec, phi_color, phi_normal, phi_depth,
                                         [&](int xx, int yy) { return __ldg(src + yy * w + xx).w; },
                                         [&](int xx, int yy) { return __ldg(edge + yy * w + xx).z; });
@@ -576,7 +583,11 @@ __global__ void __launch_bounds__(kTmaTile * kTmaTile) k_atrous_tma(const __grid
     const int ci = (ty + 2 * r) * n + (tx + 2 * r);
     const float4 center = t_src[ci];
     const float4 ec = t_edge[ci];
-    __syncthreads();
+    const bool on = x < w && y < h;
+    if (!__syncthreads_or(on && edge_material(ec) >= 0)) {  // no surface: nothing to filter
+        if (on) atrous_write(ep, dst, i, center, ec);
+        return;
+    }
     // What every tap would compute from its record, once per staged pixel.
     AtrousTile t{t_src, t_edge, t_dir};
     for (int k = ty * kTmaTile + tx; k < n * n; k += kTmaTile * kTmaTile) {
@@ -584,7 +595,7 @@ __global__ void __launch_bounds__(kTmaTile * kTmaTile) k_atrous_tma(const __grid
         t.prepare(k, t_src[k], t_edge[k], xx >= 0 && yy >= 0 && xx < w && yy < h);
     }
     __syncthreads();
-    if (x >= w || y >= h) return;
+    if (!on) return;
     // (A contiguous tile holds the pixel's neighbours too.)
     const int origin = Rank == 2 ? (2 * r - cy0) * n + 2 * r - cx0 : 0;
     const float4 result = atrous_filter(t, ci, r, r * n, x, y, w, h, step, center, ec, phi_color, phi_normal, phi_depth,
