@@ -39,19 +39,20 @@ WORKLOAD = "262,144-triangle terrain scene (value-noise height field + 200 insta
            "64 emitters, 4 punctual lights, 1024x512 HDR sky), 1920x1080, 16 spp, max depth 12, seed 1"
 # Algorithmic bytes of the traversal kernels: one 64-byte node per visit, one 48-byte triangle per test.
 NODE_BYTES, TRI_BYTES = 64, 48
-# Modelled bytes of one shaded vertex in k_shade (path state in and out, hit, shadow entry, triangle,
+# Modelled bytes of one shaded vertex (path state in and out, hit, shadow entry, triangle,
 # indices, vertex attributes, material).
 SHADE_BYTES_PER_VERTEX = 450
 # DRAM bytes (read + write) per traced ray of the closest-hit walk: its first launch in the 960x540x4
-# profile case of the same scene (photon_b200/profile_case.py; 2,073,600 camera rays, 75.03 MB read +
-# 11.30 MB written in one ncu capture), scaled by the rays of a launch here: mostly the path state
+# profile case of the same scene (photon_b200/profile_case.py; 2,073,600 camera rays, 77.11 MB read +
+# 12.74 MB written in one ncu capture), scaled by the rays of a launch here: mostly the path state
 # streaming in and the hits out; the nodes and triangles stay in L2.
-TRACE_DRAM_BYTES_PER_RAY = (75.03e6 + 11.30e6) / 2073600
-# Active threads per warp instruction (smsp__thread_inst_executed_per_inst_executed) of the pair walks
-# in the same capture (ncu --set full on python -m photon_b200.profile_case): the camera rays' launch,
-# then the first two bounces. The per-lane walks it replaced ran at 11.9 / 8.1 / 7.0 (closest hit) and
-# 7.7 / 6.1 / 5.8 (any hit) on the same case.
-NCU_THREADS_PER_INSTRUCTION = {"trace": [18.2, 15.4, 14.1], "shadow": [15.0, 13.0, 12.5], "of": 32,
+TRACE_DRAM_BYTES_PER_RAY = (77.11e6 + 12.74e6) / 2073600
+# Active threads per warp instruction (smsp__thread_inst_executed_per_inst_executed) of the list walks
+# in the same capture (ncu on python -m photon_b200.profile_case): the camera rays' launch, then the first
+# bounce. The pair walks and the per-lane walks before them on the same case: the camera rays and the first
+# two bounces.
+NCU_THREADS_PER_INSTRUCTION = {"trace": [22.6, 20.0], "shadow": [20.1, 17.7], "of": 32,
+                               "pair_walks": {"trace": [18.2, 15.4, 14.1], "shadow": [15.0, 13.0, 12.5]},
                                "per_lane_walks": {"trace": [11.9, 8.1, 7.0], "shadow": [7.7, 6.1, 5.8]}}
 # Workload description shared by both arms (the reference arm renders a bounded sample of it).
 CONFIG = {"workload": WORKLOAD, "scene_triangles": TRIS, "width": WIDTH, "height": HEIGHT, "spp": SPP, "max_depth": DEPTH,
@@ -474,15 +475,15 @@ def main():
     l2_peak = native.l2_read_bandwidth(local)
     closest_rays_frame = counts.closest_rays  # the counted render is one frame
     pairs = r.tuning()["pair_walk"] > 0
-    roofline = {"bound": "hbm", "limiter": "L2/L1 latency and issue: the scene is L2-resident (see l2, simt)",
-                "kernel": "k_trace_pairs (closest-hit BVH traversal, pair walk)" if pairs else "k_trace (closest-hit BVH traversal)",
+    roofline = {"bound": "hbm", "limiter": "issue and L1 wavefronts together: the scene is L2-resident (see l2, simt)",
+                "kernel": "k_trace_list (closest-hit BVH traversal, list walk)" if pairs else "k_trace (closest-hit BVH traversal)",
                 "l2": {"achieved": achieved, "peak": l2_peak, "unit": "GB/s", "frac": achieved / l2_peak if l2_peak > 0 else None,
                        "peak_source": "live pt_measure_l2_bandwidth: 32 MiB L2-resident buffer read 64 times per launch "
                                       "(ld.global.cg), best of 5"},
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)",
                 "traffic": TRACE_DRAM_BYTES_PER_RAY * closest_rays_frame * args.steps / trace_launches,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per traced ray of k_trace on the "
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per traced ray of k_trace_list on the "
                                   "960x540x4 profile case, times this frame's rays per launch",
                 "algorithmic_bytes_per_launch": trace_bytes_per_frame * args.steps / trace_launches,
                 "avg_launch_ms": prof.trace.ms / trace_launches,
@@ -490,23 +491,23 @@ def main():
                 "node_visits_per_ray": counts.closest_node_visits / max(1, counts.closest_rays),
                 "tri_tests_per_ray": counts.closest_tri_tests / max(1, counts.closest_rays),
                 # SIMT use of the two walks: from the counted render, the lanes that visit a node per
-                # node-visit round of a pair walk (per walk step of a per-lane walk), of 32; from the
+                # node-visit round of a pair walk, which counted renders keep (per walk step of a per-lane walk), of 32; from the
                 # profile capture, the active threads per warp instruction.
                 "simt": {"trace_lanes_per_round" if pairs else "trace_lanes_per_step": counts.closest_lane_steps / max(1, counts.closest_warp_steps),
                          "shadow_lanes_per_round" if pairs else "shadow_lanes_per_step": counts.shadow_lane_steps / max(1, counts.shadow_warp_steps),
                          "of": 32, "ncu_threads_per_instruction": NCU_THREADS_PER_INSTRUCTION},
-                "shadow": {"kernel": "k_shadow_pairs (any-hit BVH traversal, pair walk)" if pairs else "k_shadow (any-hit BVH traversal)",
+                "shadow": {"kernel": "k_shadow_list (any-hit BVH traversal, list walk)" if pairs else "k_shadow (any-hit BVH traversal)",
                            "bytes_per_frame": shadow_bytes_per_frame,
                            "ms_per_frame": prof.shadow.ms / args.steps, "achieved": shadow_achieved,
                            "l2_frac": shadow_achieved / l2_peak if l2_peak > 0 else None, "hbm_frac": shadow_achieved / peak},
-                "shade": {"kernel": "k_shade (material-sorted shading of the traced paths)",
+                "shade": {"kernel": "k_class_count, k_class_order, k_shade_misses and k_shade_ordered (the traced paths in class order)",
                           "model": f"{SHADE_BYTES_PER_VERTEX} B per shaded vertex: path state 80 B in and out, hit 16 B, "
                                    "shadow entry 48 B, triangle record, vertex indices, three vertices' attributes and "
                                    "the material (a model, not a count)",
                           "vertices_per_frame": shaded_vertices,
                           "ms_per_frame": prof.shade.ms / args.steps, "achieved": shade_achieved,
                           "hbm_frac": shade_achieved / peak,
-                          "limiter": "latency: attribute, material and texture gathers at 16 warps per SM (114 registers)"}}
+                          "limiter": "latency: attribute, material and texture gathers at 20 warps per SM (96 registers)"}}
     rays_per_sample = (counts.closest_rays + counts.shadow_rays) / samples_per_step
 
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

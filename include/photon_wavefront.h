@@ -240,16 +240,20 @@ typedef struct pt_tuning {
     int32_t shade_block;       /* threads per block of the shading kernel */
     int32_t sort_by_material;  /* k in 1-4: the shading kernel groups windows of k x shade_block paths by material
                                   class before shading them (4k x shade_block on iterations whose rays
-                                  are sorted afterwards); 0: queue order; -1 keep */
+                                  are sorted afterwards), and renders of at least 262,144 paths are
+                                  shaded in class order over the whole queue; 0: queue order; -1 keep */
     int32_t graph_bounces;     /* bounce iterations captured per CUDA graph launch */
     int32_t sort_rays;         /* 0 off, 1-6: sort continuing rays by direction octant + Morton origin cell
                                   with this many bits per axis before tracing them, on iterations of at
                                   least 2,097,152 paths (4: the renderer's default; the server: 0); -1 keep */
     int32_t packed;            /* 1: f32x2 (packed FP32) slab tests in traversal, 0: scalar; -1 keep */
     int32_t tail_paths;        /* once no new paths remain and at most this many are queued, one kernel finishes
-                                  them (a thread per path, every bounce); 0 never; -1 keep; -2 (default)
-                                  131,072 for a render that starts while no other render of this process
-                                  runs on the device, 65,536 otherwise and in the server */
+                                  them (every bounce; eight lanes per path up to 16,384 paths, else a
+                                  thread per path); 0 never; -1 keep; -2 (default) 16,384 for a render that
+                                  starts while no other render of this process runs on the device, 8,192
+                                  beside one or two others, on a scene of fewer than 512 BVH nodes and in
+                                  the server, 4,096 beside more; on trees that cannot be walked out of
+                                  order (the stack or the boxes are irregular) 131,072 and 65,536 */
     int32_t wide_shadows;      /* 1: shadow rays walk a 4-wide BVH collapsed from the scene's BVH2 (same
                                   answers), 0 (default): the BVH2; -1 keep */
     int32_t trace_refill;      /* 1-32: a warp of the closest-hit walk claims new rays for its idle lanes
@@ -262,10 +266,11 @@ typedef struct pt_tuning {
                                   2,097,152 paths ordered by direction octant + Morton origin cell (this
                                   many bits per axis); -1 keep */
     int32_t pair_walk;         /* 0: each lane walks its ray through node visits and triangle tests on its own;
-                                  1-64 (default 5): pair walks, with the leaf triangles a warp's rays reach
-                                  tested by all its lanes together after up to this many node visits per
-                                  lane (same hits and answers; packed slab tests and the BVH2 only, so
-                                  packed = 0 and the 4-wide shadow walk use the per-lane walks); -1 keep */
+                                  1-64 (default 5): the leaf triangles a warp's rays reach are tested by
+                                  all its lanes together after up to this many node visits per lane (pair
+                                  walks; list walks, which visit on meanwhile, where the tree may be walked
+                                  out of order: same hits and answers; packed slab tests and the BVH2 only,
+                                  so packed = 0 and the 4-wide shadow walk use the per-lane walks); -1 keep */
 } pt_tuning;
 int32_t pt_set_tuning(pt_renderer* r, const pt_tuning* t);
 int32_t pt_get_tuning(const pt_renderer* r, pt_tuning* t);
@@ -315,7 +320,7 @@ int32_t pt_get_profile(const pt_renderer* r, pt_profile* out);
 /* Primary closest hits of pixel centres + the first random jitter of sample `frame`, exactly the
  * camera rays of render_sample (pixel.h:18-24): per pixel (t, tri, u, v) into hits4 (4 * w * h floats;
  * tri is stored as a float bit pattern of the int32, -1 on a miss). Walked as the renderer's rendering
- * walks them: the pair walk unless its tuning sets pair_walk = 0 (or packed = 0). */
+ * walks them: the list or pair walk unless its tuning sets pair_walk = 0 (or packed = 0). */
 int32_t pt_trace_primary(pt_renderer* r, const pt_camera* camera, int32_t width, int32_t height, uint32_t frame,
                          uint32_t seed, float* hits4);
 /* The light pick of next event estimation at the first vertex of every pixel's sample `frame`
@@ -367,9 +372,9 @@ int32_t pt_svgf_run(pt_svgf* s, const float* color, const float* albedo, const f
                     const float* position, const float* emission, const pt_camera* previous,
                     const pt_svgf_settings* settings, float* output);
 /* The variance estimate of the last run (Svgf::variance_buffer, svgf.h:44): a device pointer. */
-/* How the a-trous passes read their 5x5 taps: 0 from global memory; 1 (default) from shared-memory
- * tiles that the Tensor Memory Accelerator stages, contiguous tiles for steps 1-8 and global loads
- * beyond; 2 as 1 plus a strided tile (one residue class of x, y mod 8) for step 16; 3 strided tiles
+/* How the a-trous passes read their 5x5 taps. Without this call: from shared-memory tiles that the Tensor
+ * Memory Accelerator stages for steps 1-4, and rows staged by plain loads for steps 8 and 16. 0: from
+ * global memory; 1: contiguous tiles for steps 1-8 and global loads beyond; 2 as 1 plus a strided tile (one residue class of x, y mod 8) for step 16; 3 strided tiles
  * for steps 1-16. Every mode gives the same output bit for bit. */
 int32_t pt_svgf_set_tma(pt_svgf* s, int32_t mode);
 /* Test hook for the TMA passes' bounded wait (no counterpart in Photon): with on = 1 they arm their

@@ -39,21 +39,23 @@ struct Tuning {
     int path_capacity = 1 << 24;   // paths in flight (the pool grows to what a render needs, up to this)
     int trace_block = 128;
     int shade_block = 256;
-    int sort_by_material = 4;      // shade windows of 4 x shade_block paths grouped by material class
+    int sort_by_material = 4;      // shade windows of 4 x shade_block paths grouped by material class; > 0:
+                                   // renders of at least kOrderMinPaths paths in class order over the queue
     int graph_bounces = 4;         // iterations per CUDA graph launch
     int sort_rays = 4;             // origin bits per axis of the ray-sort key (0: no sorting); iterations of
                                    // at least 2M paths only
     int packed = 1;                // f32x2 slab tests
     int wide_shadows = 0;          // 1: shadow rays walk the 4-wide BVH (measured slower on the 262K scene:
                                    // as a pair walk 13.2 ms against 11.0 per 1080p frame)
-    int tail_paths = kTailAuto;    // finish the last queued paths one thread each below this many (0: never)
+    int tail_paths = kTailAuto;    // finish the last queued paths in one kernel at or below this many (0: never)
     int trace_refill = 24;         // a closest-hit warp claims new rays once fewer than this many lanes hold one
     int shadow_refill = 24;        // the same for the shadow walk
     int walk_burst = 16;           // walk steps a lane takes between two refill checks of its warp
-    int pair_walk = 5;             // > 0: pair walks (leaf triangles of a warp tested together) with up to
-                                   // this many node visits per warp step; 0: per-lane walks. On the 262K
-                                   // scene's 1080p frame: trace 28.2 -> 24.0 ms, shadow 13.7 -> 11.0 ms
-                                   // (4 to 6 visits within noise; 2: 26.1 ms, 10: 25.6 ms)
+    int pair_walk = 5;             // > 0: the walks that test a warp's leaf triangles together, with up to this
+                                   // many node visits per warp step (pair walk; the list walk of order-free
+                                   // trees: twice as many rounds); 0: per-lane walks. On the 262K scene's
+                                   // 1080p frame: trace 28.2 (per lane), 23.5 (pairs), 21.1 ms (lists), shadow
+                                   // 13.7, 10.9, 9.6 (pairs: 4 to 6 visits within noise; 2: 26.1 ms, 10: 25.6)
     int sort_shadows = 0;          // origin bits per axis of the shadow-queue walk order (0: queue order);
                                    // iterations of at least 2M paths only. Off: on the 262K scene's 1080p
                                    // frame the shadow walk took 13.65 ms sorted against 13.63 unsorted (the
