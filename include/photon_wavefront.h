@@ -323,6 +323,13 @@ int32_t pt_get_profile(const pt_renderer* r, pt_profile* out);
  * walks them: the list or pair walk unless its tuning sets pair_walk = 0 (or packed = 0). */
 int32_t pt_trace_primary(pt_renderer* r, const pt_camera* camera, int32_t width, int32_t height, uint32_t frame,
                          uint32_t seed, float* hits4);
+/* How the uploaded scene is walked by default: *order_free 1 if its tree may be walked out of order (list
+ * walks; else walks in Photon's order), *group_tail 1 if small tails walk it by groups of eight lanes. */
+int32_t pt_scene_walks(const pt_renderer* r, int32_t* order_free, int32_t* group_tail);
+/* The levels of a BVH of num_nodes nodes as an upload counts them: 0 where a node has two parents (the scene
+ * is accepted and walked in Photon's order), 255 for 255 and more, -1 where a child does not follow its
+ * parent or is out of range (the scene is refused). Needs no device. */
+int32_t pt_bvh_levels(const pt_bvh_node* nodes, int32_t num_nodes);
 /* The light pick of next event estimation at the first vertex of every pixel's sample `frame`
  * (integrator.h:206-209 with lights.h:139-202): per pixel 4 int32 = group (0 emissive, 1 punctual,
  * 2 environment, -1 none), index (emissive entry, punctual light, or env row*width+col), alias bin,

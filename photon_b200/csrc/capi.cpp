@@ -246,6 +246,22 @@ int32_t pt_trace_primary(pt_renderer* r, const pt_camera* camera, int32_t width,
     PT_RENDERER_CALL(r, r->r->trace_primary(*camera, width, height, frame, seed, hits4));
 }
 
+int32_t pt_scene_walks(const pt_renderer* r, int32_t* order_free, int32_t* group_tail) {
+    if (!r || !r->r || !order_free || !group_tail) return PT_ERR_INVALID;
+    r->r->scene_walks(order_free, group_tail);
+    return PT_OK;
+}
+
+int32_t pt_bvh_levels(const pt_bvh_node* nodes, int32_t num_nodes) {
+    if (!nodes || num_nodes < 1) return -1;
+    for (int32_t i = 0; i < num_nodes; i++) {
+        const pt_bvh_node& b = nodes[i];
+        if (b.lcount <= 0 && b.left >= 0 && (b.left <= i || b.left >= num_nodes)) return -1;
+        if (b.rcount <= 0 && b.right >= 0 && (b.right <= i || b.right >= num_nodes)) return -1;
+    }
+    return bvh_levels(nodes, num_nodes);
+}
+
 int32_t pt_light_picks_primary(pt_renderer* r, const pt_camera* camera, const pt_render_settings* settings, uint32_t frame, int32_t* picks4) {
     if (!camera || !settings || !picks4) return PT_ERR_INVALID;
     PT_RENDERER_CALL(r, r->r->light_picks(*camera, *settings, frame, picks4));

@@ -77,6 +77,25 @@ void validate_scene(const pt_scene_desc& d, bool lights_only) {
     }
 }
 
+int bvh_levels(const pt_bvh_node* nodes, int32_t n) {
+    std::vector<uint8_t> level(size_t(n), 0);  // 0: no parent so far
+    level[0] = 1;
+    int most = 1;
+    for (int32_t i = 0; i < n; i++) {
+        const pt_bvh_node& b = nodes[i];
+        const int32_t idx[2] = {b.left, b.right}, cnt[2] = {b.lcount, b.rcount};
+        const int next = std::min(std::max<int>(level[size_t(i)], 1) + 1, 255);
+        for (int k = 0; k < 2; k++) {
+            if (cnt[k] > 0 || idx[k] < 0) continue;
+            uint8_t& l = level[size_t(idx[k])];
+            if (l) return 0;
+            l = uint8_t(next);
+            most = std::max(most, next);
+        }
+    }
+    return most;
+}
+
 size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
     size_t b = 0;
     b += size_t(d.num_nodes) * 64 + size_t(d.num_tris) * (16 * kTriStride + 16);
@@ -130,15 +149,7 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
         } else {
             nodes4_.release();
         }
-        // Levels of the tree (children follow their parents).
-        std::vector<uint8_t> level(size_t(d.num_nodes), 1);
-        tree_depth_ = 1;
-        for (int32_t i = 0; i < d.num_nodes; i++) {
-            const uint8_t next = uint8_t(std::min<int>(level[size_t(i)] + 1, 255));
-            tree_depth_ = std::max<int>(tree_depth_, level[size_t(i)]);
-            if (d.nodes[i].lcount <= 0 && d.nodes[i].left >= 0) level[size_t(d.nodes[i].left)] = next;
-            if (d.nodes[i].rcount <= 0 && d.nodes[i].right >= 0) level[size_t(d.nodes[i].right)] = next;
-        }
+        tree_levels_ = bvh_levels(d.nodes, d.num_nodes);
         num_vertices_ = d.num_vertices;
         if (d.normals) {
             std::vector<float4> n(size_t(d.num_vertices));
@@ -247,13 +258,13 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.p_emissive = d.p_emissive;
     v.p_punctual = d.p_punctual;
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
-    v.bvh_depth = tree_depth_;
+    v.bvh_depth = tree_levels_;
     try {
-        v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_depth_, s) ? 1 : 0;
+        v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_levels_, s) ? 1 : 0;
         if (!v.order_free) {
             wide_.release();
         } else if (!lights_only || !wide_.ptr) {
-            wide_tree_build(nodes_.ptr, v.num_nodes, tree_depth_, wide_, s);
+            wide_tree_build(nodes_.ptr, v.num_nodes, tree_levels_, wide_, s);
         }
     } catch (const Error&) {
         // No memory for the 8-wide tree: the scene is walked in Photon's order, which needs none. (Any other

@@ -105,12 +105,17 @@ private:
     float extent_ = 1.0f;
     int32_t num_vertices_ = 0;
     int32_t num_materials_ = 0;
-    int tree_depth_ = 0;
+    int tree_levels_ = 0;  // bvh_levels of the uploaded tree
     void upload_shade_keys(const pt_material* materials, int32_t n, cudaStream_t s);
     float bounds_[6] = {0, 0, 0, 0, 0, 0};  // the scene box (lo xyz, hi xyz), for the light-group weights
 };
 
 // Checks a scene description for internal consistency; throws Error(PT_ERR_INVALID).
 void validate_scene(const pt_scene_desc& d, bool lights_only);
+
+// The levels of a BVH whose children follow their parents (255 and more: 255), or 0 where two parents name
+// one node, which validate_scene lets through: the walks in Photon's order take such a graph as it is, but
+// what counts on a tree's depth or on its number of nodes does not.
+int bvh_levels(const pt_bvh_node* nodes, int32_t n);
 
 }  // namespace ptw

@@ -196,6 +196,10 @@ public:
     void autotune_views(const pt_view* views, int n, uint64_t probe_samples, pt_tuning* chosen, double* default_rate, double* tuned_rate);
 
     void trace_primary(const pt_camera& cam, int w, int h, uint32_t frame, uint32_t seed, float* hits4);
+    void scene_walks(int32_t* order_free, int32_t* group_tail) const {
+        *order_free = scene_.view().order_free;
+        *group_tail = scene_.view().order_free && scene_.view().wide ? 1 : 0;
+    }
     void light_picks(const pt_camera& cam, const pt_render_settings& rs, uint32_t frame, int32_t* picks4);
     void heatmap(const pt_camera& cam, int w, int h, float* out);
     void occlusion_probe(const float* rays8, int n, int wide, int32_t* out4);

@@ -53,9 +53,9 @@ __global__ void __launch_bounds__(256) k_check_tree(const float4* __restrict__ n
 
 }  // namespace
 
-bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int depth, cudaStream_t stream) {
+bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, cudaStream_t stream) {
     // A list entry keeps 2 * node + side in 27 bits.
-    if (depth > kOrderFreeDepth || num_nodes < 1 || num_nodes >= (1 << 26)) return false;
+    if (levels < 1 || levels > kOrderFreeDepth || num_nodes < 1 || num_nodes >= (1 << 26)) return false;
     DeviceBuffer<int> bad;
     bad.allocate(1);
     bad.zero(stream);

@@ -8,8 +8,8 @@ namespace ptw {
 constexpr int kOrderFreeDepth = 60;  // levels of the tree: Photon's 64-entry stack then never drops a node
 
 // True when every box of the device-resident tree is finite, ordered and inside its parent's, every leaf's
-// triangles lie inside its box (to rounding), the tree is at most kOrderFreeDepth levels deep (`depth`:
-// its levels) and its nodes fit the list walk's entries. Synchronises the stream.
-bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int depth, cudaStream_t stream);
+// triangles lie inside its box (to rounding), no node has two parents and the tree is at most kOrderFreeDepth
+// levels deep (`levels`: bvh_levels of it), and its nodes fit the list walk's entries. Synchronises the stream.
+bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, cudaStream_t stream);
 
 }  // namespace ptw

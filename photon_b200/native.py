@@ -69,6 +69,8 @@ def _load():
         "pt_server_close_session": ([C.c_void_p, C.c_int32], C.c_int32),
         "pt_server_fetch_encoded": ([C.c_void_p, C.c_uint64, C.c_int32, C.c_void_p, C.c_size_t, P(C.c_size_t)], C.c_int32),
         "pt_trace_primary": ([C.c_void_p, P(abi.Camera), C.c_int32, C.c_int32, C.c_uint32, C.c_uint32, _f32p], C.c_int32),
+        "pt_scene_walks": ([C.c_void_p, P(C.c_int32), P(C.c_int32)], C.c_int32),
+        "pt_bvh_levels": ([C.c_void_p, C.c_int32], C.c_int32),
         "pt_light_picks_primary": ([C.c_void_p, P(abi.Camera), P(abi.RenderSettings), C.c_uint32, _i32p], C.c_int32),
         "pt_heatmap": ([C.c_void_p, P(abi.Camera), C.c_int32, C.c_int32, _f32p], C.c_int32),
         "pt_occlusion_probe": ([C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p], C.c_int32),
@@ -284,6 +286,12 @@ class Renderer:
         out = np.zeros((h, w, 4), np.float32)
         _check(lib.pt_trace_primary(self.h, C.byref(cam), w, h, frame, seed, out), self._err)
         return out
+
+    def scene_walks(self):
+        """(order_free, group_tail) of the uploaded scene (pt_scene_walks)."""
+        a, b = C.c_int32(), C.c_int32()
+        _check(lib.pt_scene_walks(self.h, C.byref(a), C.byref(b)), self._err)
+        return a.value, b.value
 
     def light_picks(self, cam, rs, frame=0):
         out = np.zeros((rs.height, rs.width, 4), np.int32)
