@@ -46,6 +46,7 @@ WavefrontEngine::WavefrontEngine(int device, cudaStream_t stream) : device_(devi
     std::memset(h_ctr_, 0, sizeof(Counters));
     PTW_CUDA(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
     ctr_.allocate(1);
+    class_ctr_.allocate(128);
 }
 
 WavefrontEngine::~WavefrontEngine() {
@@ -118,15 +119,6 @@ void WavefrontEngine::reserve_paths(uint64_t needed) {
     keys_.allocate(want);
     shadow_keys_.allocate(want);
     shadow_perm_.allocate(want);
-    try {
-        order_.allocate(want);
-        classes_.allocate(want);
-        class_ctr_.allocate(128);
-    } catch (const Error&) {  // no memory for the class order: k_shade's windows, which need none
-        cudaGetLastError();
-        order_.release();
-        classes_.release();
-    }
     pb_.capacity = uint32_t(want);
     if (graph_) {
         cudaGraphExecDestroy(graph_);
@@ -141,16 +133,13 @@ void WavefrontEngine::release_paths() {
     }
     for (auto& b : bufs_) b.release();
     for (auto& b : ids_) b.release();
-    for (DeviceBuffer<uint32_t>* b : {&keys_, &hist_, &offsets_, &shadow_keys_, &shadow_hist_, &shadow_offsets_, &shadow_perm_, &order_, &class_ctr_}) b->release();
-    classes_.release();
+    for (DeviceBuffer<uint32_t>* b : {&keys_, &hist_, &offsets_, &shadow_keys_, &shadow_hist_, &shadow_offsets_, &shadow_perm_}) b->release();
     pb_ = PathBuffers{};
 }
 
-size_t WavefrontEngine::extra_bytes() const { return order_.bytes() + classes_.bytes() + class_ctr_.bytes(); }
-
 size_t WavefrontEngine::device_bytes() const {
     size_t b = ctr_.bytes() + keys_.bytes() + hist_.bytes() + offsets_.bytes() + shadow_keys_.bytes() + shadow_hist_.bytes() +
-               shadow_offsets_.bytes() + shadow_perm_.bytes() + order_.bytes() + class_ctr_.bytes() + classes_.bytes();
+               shadow_offsets_.bytes() + shadow_perm_.bytes();
     for (const auto& x : bufs_) b += x.bytes();
     for (const auto& x : ids_) b += x.bytes();
     return b;
@@ -199,8 +188,10 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
     p.packed = tuning_.packed ? 1 : 0;
     p.sort_bits = tuning_.sort_rays;
     p.sort_material = tuning_.sort_by_material;
-    p.order = tuning_.sort_by_material > 0 ? order_.ptr : nullptr;
-    p.classes = classes_.ptr;
+    // (The class order lives between the trace and the shading, the shadow queue's keys and order from the
+    // shading to the shadow walk: they share their memory.)
+    p.order = tuning_.sort_by_material > 0 ? shadow_perm_.ptr : nullptr;
+    p.classes = reinterpret_cast<uint8_t*>(shadow_keys_.ptr);
     p.class_ctr = class_ctr_.ptr;
     p.tail_paths = tuning_.tail_paths == kTailAuto ? 1u : uint32_t(std::max(0, tuning_.tail_paths));
     p.wide_shadows = tuning_.wide_shadows;

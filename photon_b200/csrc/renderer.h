@@ -108,7 +108,7 @@ public:
         cont_params_.shadow_sort_bits = on ? tuning_.sort_shadows : 0;
     }
     // Continuous mode: whether the next launches shade in class order over the whole queue.
-    void set_continuous_ordering(bool on) { cont_params_.order = on && tuning_.sort_by_material > 0 ? order_.ptr : nullptr; }
+    void set_continuous_ordering(bool on) { cont_params_.order = on && tuning_.sort_by_material > 0 ? shadow_perm_.ptr : nullptr; }
     // Continuous mode: takes the knobs of `t` that only change what the next launches are given
     // (material-sort window, ray-sort bits up to those the buffers were sized for, packed slab tests,
     // 4-wide shadow BVH, walk refill and burst). Pool size, block shapes, graph cadence and the tail
@@ -132,7 +132,6 @@ public:
     double kernel_ms[5] = {0, 0, 0, 0, 0};
     uint64_t kernel_launches = 0, iteration_launches = 0;
     size_t device_bytes() const;
-    size_t extra_bytes() const;  // of these, what a render can do without (the shading order)
     int device() const { return device_; }
     cudaStream_t stream() const { return stream_; }
     uint64_t bytes_per_path() const;
@@ -152,8 +151,7 @@ private:
     DeviceBuffer<uint4> ids_[2];
     DeviceBuffer<Counters> ctr_;
     DeviceBuffer<uint32_t> keys_, hist_, offsets_;
-    DeviceBuffer<uint32_t> order_, class_ctr_;
-    DeviceBuffer<uint8_t> classes_;
+    DeviceBuffer<uint32_t> class_ctr_;  // (512 bytes, not counted in device_bytes)
     DeviceBuffer<uint32_t> shadow_keys_, shadow_hist_, shadow_offsets_, shadow_perm_;
     Counters* h_ctr_ = nullptr;
     Counters last_{};

@@ -51,9 +51,7 @@ Server::Server(const pt_server_config& cfg) : cfg_(cfg), device_(cfg.device) {
     created_sort_rays_ = t.sort_rays;
     engine_->set_tuning(t);
     engine_->reserve_paths(uint64_t(t.path_capacity));
-    // The budget admits by what rendering needs: the extras (5 bytes per path, up to 96 per BVH node; given up
-    // where memory runs out) take no request's place.
-    pool_bytes_ = engine_->device_bytes() - engine_->extra_bytes();
+    pool_bytes_ = engine_->device_bytes();
     d_scenes_.allocate(kMaxScenes);
     d_views_.allocate(1024);
     d_done_.allocate(1024);
@@ -91,7 +89,7 @@ Server::Server(const pt_server_config& cfg) : cfg_(cfg), device_(cfg.device) {
         Tuning st;
         st.path_capacity = 1 << 23;  // grown on the first frames to what they need, up to this
         session_engine_->set_tuning(st);
-        lane_idle_bytes_ = session_engine_->device_bytes() - session_engine_->extra_bytes();
+        lane_idle_bytes_ = session_engine_->device_bytes();
     }
     for (Batch& b : batch_) {
         PTW_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&b.ctr), sizeof(Counters), cudaHostAllocDefault));
@@ -578,7 +576,7 @@ void Server::session_loop() {
         }
 
         lk.lock();
-        size_t lane = session_engine_->device_bytes() - session_engine_->extra_bytes() - lane_idle_bytes_;
+        size_t lane = session_engine_->device_bytes() - lane_idle_bytes_;
         pool_bytes_ = pool_bytes_ - lane_bytes_ + lane;
         lane_bytes_ = lane;
         for (Request* r : frames) {

@@ -101,8 +101,9 @@ struct WfParams {
     int order_free;            // 1: every scene of the launch is DevScene::order_free, so that the walks with
                                //    pair_visits > 0 are list walks (uncounted launches)
     int sort_material;         // 1: the shade kernel groups each block's paths by material class
-    uint32_t* order;           // capacity entries: the shade order by class, or null (shaded by k_shade)
-    uint8_t* classes;          // capacity entries: their shading classes
+    uint32_t* order;           // capacity entries: the shade order by class, or null (shaded by k_shade). Read up to
+                               // the end of the shading; its memory is shadow_perm's
+    uint8_t* classes;          // capacity entries: their shading classes, read before the shading; shadow_keys' memory
     uint32_t* class_ctr;       // per class: paths of the iteration, then paths placed in the order
     int sort_bits;             // > 0: sort continuing paths by direction octant + Morton origin cell
                                //      (this many bits per axis) before they are traced

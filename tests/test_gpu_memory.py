@@ -1,0 +1,47 @@
+"""What scenes and path pools hold on the device is what the server counts (its budget bounds it), and buffers
+that share memory hold the right thing at the right time."""
+import numpy as np
+import pytest
+
+from photon_b200 import abi, native
+
+pytestmark = pytest.mark.gpu
+SLACK = 12 << 20  # the counted arrays round up to whole device pages; the context's own growth
+
+
+@pytest.fixture(scope="module")
+def cuda():
+    return pytest.importorskip("torch").cuda
+
+
+def _free(cuda):
+    cuda.synchronize()
+    return cuda.mem_get_info()[0]
+
+
+def test_a_path_pool_holds_what_is_counted(cuda):
+    native.Server(path_capacity=1 << 20, reserve_bytes=-1).close()  # the context and its modules
+    before = _free(cuda)
+    s = native.Server(path_capacity=1 << 24, reserve_bytes=-1)
+    held, counted = before - _free(cuda), s.stats().device_bytes_in_use
+    s.close()
+    assert counted > 1 << 30
+    assert held <= counted + SLACK
+
+
+@pytest.mark.parametrize("kind", ["box", "terrain"])
+def test_the_class_order_beside_sorted_shadow_rays(kind):
+    """The order of the shading and that of the shadow walk share their memory: an iteration that has both."""
+    g = native.box_scene() if kind == "box" else native.terrain_scene(65536, 3)
+    b = g.build()
+    w, h = 2048, 1026  # above the 2^21 paths from which rays are sorted
+    cam, out = g.camera(w / h), []
+    for t in (dict(sort_by_material=0, sort_rays=0), dict(sort_shadows=4)):
+        r = native.Renderer()
+        r.upload(b.desc)
+        r.resize(w, h)
+        r.set_tuning(**t)
+        r.render(cam, abi.render_settings(w, h, max_depth=4, seed=2), 1)
+        out.append(r.download_accumulation())
+        r.close()
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
