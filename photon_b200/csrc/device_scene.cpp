@@ -7,8 +7,8 @@
 // luminance of each environment texel (math.h:112), so the device never needs those transcendentals.
 #include "device_scene.h"
 #include "tree_check.h"
+#include "treelets.h"
 #include "wide_bvh.h"
-#include "wide_tree.h"
 
 #include <algorithm>
 #include <cmath>
@@ -106,10 +106,8 @@ size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
     return b + sizeof(DevScene);
 }
 
-size_t DeviceScene::extra_bytes() const { return wide_.bytes() + light_work_.bytes(); }
-
 size_t DeviceScene::device_bytes() const {
-    return nodes_.bytes() + nodes4_.bytes() + wide_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
+    return nodes_.bytes() + nodes4_.bytes() + tris_.bytes() + normals_.bytes() + tangents_.bytes() + materials_.bytes() + alias_.bytes() +
            punctual_.bytes() + env_texels_.bytes() + tri_idx_.bytes() + textures_.bytes() + uvs_.bytes() + texels_.bytes() +
            srgb_lut_.bytes() + env_marginal_.bytes() + env_conditional_.bytes() + env_row_sin_.bytes() + emissive_.bytes() +
            shade_keys_.bytes() + light_work_.bytes() + d_view_.bytes();
@@ -138,6 +136,7 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     if (lights_only && d.num_tris != view_.num_tris) throw Error{PT_ERR_INVALID, "update_lights: the triangle count changed"};
     validate_scene(d, lights_only);
     if (!lights_only) {
+        d_view_.allocate(1);
         nodes_.upload(reinterpret_cast<const float4*>(d.nodes), size_t(d.num_nodes) * 4, s);
         // The 4-wide BVH for any-hit rays, collapsed from the same tree (absent if it does not fit
         // the walk's stack or leaf encoding; the shadow rays then walk the BVH2).
@@ -149,7 +148,11 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
         } else {
             nodes4_.release();
         }
+        // In treelet order for the tail by groups of lanes, before the other arrays take memory: the copy that
+        // this needs for a moment is no more than they will.
         tree_levels_ = bvh_levels(d.nodes, d.num_nodes);
+        const bool shallow = tree_levels_ > 0 && tree_levels_ <= kOrderFreeDepth;
+        root_treelet_ = shallow ? order_by_treelets(nodes_, d.num_nodes, tree_levels_, reinterpret_cast<int*>(d_view_.ptr), s) : 0;
         num_vertices_ = d.num_vertices;
         if (d.normals) {
             std::vector<float4> n(size_t(d.num_vertices));
@@ -259,21 +262,8 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.p_punctual = d.p_punctual;
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
     v.bvh_depth = tree_levels_;
-    try {
-        v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_levels_, s) ? 1 : 0;
-        if (!v.order_free) {
-            wide_.release();
-        } else if (!lights_only || !wide_.ptr) {
-            wide_tree_build(nodes_.ptr, v.num_nodes, tree_levels_, wide_, s);
-        }
-    } catch (const Error&) {
-        // No memory for the 8-wide tree: the scene is walked in Photon's order, which needs none. (Any other
-        // failure shows again at the synchronisation that ends the upload.)
-        cudaGetLastError();
-        wide_.release();
-        v.order_free = 0;
-    }
-    v.wide = wide_.ptr;
+    v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_levels_, reinterpret_cast<int*>(d_view_.ptr), s) ? 1 : 0;
+    v.root_treelet = v.order_free ? root_treelet_ : 0;
     {
         float lo[3] = {d.bounds_min.x, d.bounds_min.y, d.bounds_min.z}, hi[3] = {d.bounds_max.x, d.bounds_max.y, d.bounds_max.z};
         float inv[3];

@@ -55,6 +55,21 @@ struct DeviceBuffer {
         PTW_CUDA(cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T)));
         count = n;
     }
+    // allocate() for what can be done without: false, with nothing held, where there is no memory for it.
+    bool try_allocate(size_t n) {
+        if (n == count && ptr) return true;
+        release();
+        if (n == 0) return true;
+        const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            ptr = nullptr;
+            return false;
+        }
+        PTW_CUDA(e);
+        count = n;
+        return true;
+    }
     // Grows (never shrinks) to at least n elements; returns true when the allocation changed.
     bool reserve(size_t n) {
         if (n <= count && ptr) return false;
@@ -81,8 +96,6 @@ public:
     const DevScene* device_view() const { return d_view_.ptr; }
     bool ready() const { return ready_; }
     size_t device_bytes() const;
-    // Of these, what a render can do without (the 8-wide tree, the light rebuild's scratch).
-    size_t extra_bytes() const;
     float extent() const { return extent_; }
     // Bytes a scene will occupy on the device (for admission before upload).
     static size_t estimate_bytes(const pt_scene_desc& d);
@@ -91,7 +104,7 @@ public:
     void rebuild_lights(const pt_light_update& u, cudaStream_t stream);
 
 private:
-    DeviceBuffer<float4> nodes4_, wide_;
+    DeviceBuffer<float4> nodes4_;
     DeviceBuffer<float4> nodes_, tris_, normals_, tangents_, materials_, alias_, punctual_, env_texels_;
     DeviceBuffer<int4> tri_idx_, textures_;
     DeviceBuffer<float2> uvs_;
@@ -105,7 +118,8 @@ private:
     float extent_ = 1.0f;
     int32_t num_vertices_ = 0;
     int32_t num_materials_ = 0;
-    int tree_levels_ = 0;  // bvh_levels of the uploaded tree
+    int tree_levels_ = 0;   // bvh_levels of the uploaded tree
+    int root_treelet_ = 0;  // order_by_treelets of it, 0 if it keeps the order it came in
     void upload_shade_keys(const pt_material* materials, int32_t n, cudaStream_t s);
     float bounds_[6] = {0, 0, 0, 0, 0, 0};  // the scene box (lo xyz, hi xyz), for the light-group weights
 };

@@ -15,6 +15,14 @@ namespace ptw {
 constexpr int kStackSize = 64;     // Photon's kStackSize (traverse.h:22)
 constexpr int kSmemStack = 16;     // entries per thread kept in shared memory
 
+// The walks that test leaves later than Photon does (the list walk, the group walk) prune at kPrune times the
+// least distance so far, and leave a ray to Photon's walk if they accept a triangle nearer than kAhead times
+// its leaf box's entry, or a second one within kNearTie times the least distance. (1 / kAhead is below kNearTie
+// by more than the products' rounding. A kNearTie of 1 + 2^-13, which would do too, cost 0.4% of a frame.)
+constexpr float kPrune = 1.0f + 1.0f / 1024.0f;
+constexpr float kNearTie = 1.0f + 1.0f / 16384.0f;
+constexpr float kAhead = 1.0f - 63.0f / 64.0f / 16384.0f;
+
 struct Hit {
     float t;
     int tri;

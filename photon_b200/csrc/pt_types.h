@@ -23,7 +23,6 @@ constexpr int kTriStride = 4;
 struct DevScene {
     const float4* nodes;
     const float4* nodes4;     // the 4-wide BVH for any-hit rays (8 float4 per node), or null
-    const float4* wide;       // the group walk's 8-wide tree (wide_tree.h), or null unless order_free
     const float4* tris;
     const int4* tri_idx;
     const float4* normals;
@@ -49,7 +48,8 @@ struct DevScene {
     float p_env, p_emissive, p_punctual;
     int has_lights;
     int bvh_depth;
-    int order_free;  // 1: the tree may be walked out of order (tree_is_order_free)
+    int order_free;    // 1: the tree may be walked out of order (tree_is_order_free)
+    int root_treelet;  // > 0: order_free, with its nodes in treelet order; the size of the root's treelet
     float bounds_lo_x, bounds_lo_y, bounds_lo_z;   // scene box (for ray-sort keys)
     float inv_extent_x, inv_extent_y, inv_extent_z;
 };

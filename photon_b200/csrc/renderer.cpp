@@ -195,7 +195,7 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
     p.class_ctr = class_ctr_.ptr;
     p.tail_paths = tuning_.tail_paths == kTailAuto ? 1u : uint32_t(std::max(0, tuning_.tail_paths));
     p.wide_shadows = tuning_.wide_shadows;
-    p.group_tail = p.order_free && !count && tuning_.packed && tuning_.pair_walk > 0 ? kGroupTail : 0u;
+    p.group_tail = count ? 0u : single >= 0 ? group_tail(single_host->order_free, single_host->root_treelet > 0) : group_tail(order_free_, treelets_);
     p.trace_refill = uint32_t(std::clamp(tuning_.trace_refill, 1, 32));
     p.shadow_refill = uint32_t(std::clamp(tuning_.shadow_refill, 1, 32));
     p.walk_burst = uint32_t(std::clamp(tuning_.walk_burst, 1, 1 << 20));
@@ -286,6 +286,27 @@ void WavefrontEngine::run(const DevScene* scenes, int single_scene, const DevSce
     last_ = *h_ctr_;
 }
 
+uint32_t WavefrontEngine::group_tail(bool order_free, bool treelets) const {
+    return order_free && treelets && tuning_.packed && tuning_.pair_walk > 0 ? kGroupTail : 0u;
+}
+
+// Continuous mode: the tail's threshold for the walk that tails take now (a server shares the GPU between
+// requests), onto the device.
+void WavefrontEngine::set_tail_limit() {
+    const uint32_t limit = tail_limit(tuning_.tail_paths, cont_params_.group_tail > 0, false, 1);
+    if (!cont_params_.ctr || limit == tail_limit_) return;
+    h_ctr_->tail_limit = tail_limit_ = limit;
+    PTW_CUDA(cudaMemcpyAsync(&ctr_.ptr->tail_limit, &h_ctr_->tail_limit, sizeof(uint32_t), cudaMemcpyHostToDevice, stream_));
+}
+
+void WavefrontEngine::set_scenes(const std::vector<DevScene>& table) {
+    order_free_ = std::all_of(table.begin(), table.end(), [](const DevScene& s) { return s.order_free != 0; });
+    treelets_ = std::all_of(table.begin(), table.end(), [](const DevScene& s) { return s.root_treelet > 0; });
+    cont_params_.order_free = order_free_ ? 1 : 0;
+    cont_params_.group_tail = group_tail(order_free_, treelets_);
+    set_tail_limit();
+}
+
 void WavefrontEngine::begin(const DevScene* scenes, const DevView* views, int n_views) {
     ensure_shape();
     std::memset(h_ctr_, 0, sizeof(Counters));
@@ -316,6 +337,7 @@ void WavefrontEngine::update_scheduling(const Tuning& t) {
     cont_params_.walk_burst = fresh.walk_burst;
     cont_params_.pair_visits = fresh.pair_visits;
     cont_params_.group_tail = fresh.group_tail;
+    set_tail_limit();
     if (cont_params_.sort_bits > 0) cont_params_.sort_bits = tuning_.sort_rays;
 }
 

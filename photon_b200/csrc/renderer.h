@@ -115,12 +115,8 @@ public:
     // stay as they were set before begin().
     void update_scheduling(const Tuning& t);
 
-    // Whether every scene that multi-scene launches may meet is DevScene::order_free.
-    void set_order_free(bool all) {
-        order_free_ = all;
-        cont_params_.order_free = all ? 1 : 0;
-        if (!all) cont_params_.group_tail = 0;
-    }
+    // What every scene that multi-scene launches may meet allows.
+    void set_scenes(const std::vector<DevScene>& table);
 
     const Counters& last() const { return last_; }
 
@@ -161,7 +157,9 @@ private:
     cudaEvent_t ev_ = nullptr;
     // continuous mode
     WfParams cont_params_{};
-    bool order_free_ = false;
+    bool order_free_ = false, treelets_ = false;  // set_scenes: every scene has them
+    uint32_t group_tail(bool order_free, bool treelets) const;
+    void set_tail_limit();
     int profile_flags_ = 0;
     std::vector<cudaEvent_t> prof_ev_;
     uint32_t tail_limit_ = 0;
@@ -196,7 +194,7 @@ public:
     void trace_primary(const pt_camera& cam, int w, int h, uint32_t frame, uint32_t seed, float* hits4);
     void scene_walks(int32_t* order_free, int32_t* group_tail) const {
         *order_free = scene_.view().order_free;
-        *group_tail = scene_.view().order_free && scene_.view().wide ? 1 : 0;
+        *group_tail = scene_.view().root_treelet > 0 ? 1 : 0;
     }
     void light_picks(const pt_camera& cam, const pt_render_settings& rs, uint32_t frame, int32_t* picks4);
     void heatmap(const pt_camera& cam, int w, int h, float* out);

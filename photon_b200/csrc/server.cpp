@@ -173,10 +173,9 @@ int32_t Server::add_scene(const pt_scene_desc& d) {
     // Checked again under the lock that publishes the scene: concurrent add_scene calls all passed the
     // first check before any of them was counted, and the device scene table holds kMaxScenes entries.
     if (int(scenes_.size()) >= kMaxScenes) throw Error{PT_ERR_BUDGET, "too many resident scenes"};
-    const size_t bytes = scene->device_bytes() - scene->extra_bytes();
-    if (cfg_.budget_bytes && bytes_in_use_ + pool_bytes_ + scene_bytes_ + bytes > cfg_.budget_bytes)
+    if (cfg_.budget_bytes && bytes_in_use_ + pool_bytes_ + scene_bytes_ + scene->device_bytes() > cfg_.budget_bytes)
         throw Error{PT_ERR_BUDGET, "the scene does not fit the device-memory budget"};
-    scene_bytes_ += bytes;
+    scene_bytes_ += scene->device_bytes();
     scenes_.push_back(std::move(scene));
     scenes_dirty_ = true;
     st_.scenes = int(scenes_.size());
@@ -552,7 +551,7 @@ void Server::session_loop() {
                                      session_stream_));
             PTW_CUDA(cudaMemcpyAsync(session_views_.ptr, views.data(), views.size() * sizeof(DevView), cudaMemcpyHostToDevice,
                                      session_stream_));
-            session_engine_->set_order_free(std::all_of(table.begin(), table.end(), [](const DevScene& t) { return t.order_free != 0; }));
+            session_engine_->set_scenes(table);
             session_engine_->run(session_scenes_.ptr, single, single >= 0 ? &table[size_t(single)] : nullptr, session_views_.ptr,
                                  int(views.size()), work);
             for (size_t k = 0; k < frames.size(); k++) {
@@ -673,7 +672,7 @@ void Server::upload_scene_table() {
     std::vector<DevScene> table;
     for (const auto& s : scenes_) table.push_back(s->view());
     PTW_CUDA(cudaMemcpyAsync(d_scenes_.ptr, table.data(), table.size() * sizeof(DevScene), cudaMemcpyHostToDevice, stream_));
-    engine_->set_order_free(std::all_of(table.begin(), table.end(), [](const DevScene& s) { return s.order_free != 0; }));
+    engine_->set_scenes(table);
     scenes_dirty_ = false;
 }
 

@@ -9,7 +9,8 @@ constexpr int kOrderFreeDepth = 60;  // levels of the tree: Photon's 64-entry st
 
 // True when every box of the device-resident tree is finite, ordered and inside its parent's, every leaf's
 // triangles lie inside its box (to rounding), no node has two parents and the tree is at most kOrderFreeDepth
-// levels deep (`levels`: bvh_levels of it), and its nodes fit the list walk's entries. Synchronises the stream.
-bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, cudaStream_t stream);
+// levels deep (`levels`: bvh_levels of it), and its nodes fit the list walk's entries. `word`: an int of device
+// scratch. Synchronises the stream.
+bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, int* word, cudaStream_t stream);
 
 }  // namespace ptw

@@ -489,8 +489,6 @@ constexpr uint32_t kListVisits = 2; // rounds per step, per node visit of a pair
 // Frames of the 262K terrain, depth 8, 32 rays to a warp against this: 57,600 paths 0.933 -> 0.842 ms, 115,200
 // 1.19 -> 1.06, 230,400 1.46 -> 1.36, 1.44M 3.21 -> 3.14 (with 4 or 12 within 1% of that).
 constexpr uint32_t kListShare = 8;
-constexpr float kPrune = 1.0f + 1.0f / 1024.0f;
-constexpr float kNearTie = 1.0f + 1.0f / 16384.0f;
 
 template <bool AnyHit, bool Single>
 struct ListSlots {
@@ -546,7 +544,7 @@ __device__ __forceinline__ void list_test(ListSlots<AnyHit, Single>& ls, bool on
                 key = (unsigned long long)__float_as_uint(t) << 32 | uint32_t(i);
                 const unsigned long long old = atomicMin(&ls.best[k], key);
                 const unsigned long long other = old > key ? old : key;
-                if (t < entry * (1.0f - 1.0f / 16384.0f)) atomicMin(&ls.mark[k], 0u);
+                if (t < entry * kAhead) atomicMin(&ls.mark[k], 0u);
                 else if (other != ~0ull) atomicMin(&ls.mark[k], uint32_t(other >> 32));
             }
         }
@@ -1306,7 +1304,7 @@ __global__ void __launch_bounds__(128, 5) k_shade_ordered(const __grid_constant_
 // the queued kernels (emission, then the light sample's contribution, then the next bounce), so each
 // path's result is the same as through the queues. What bounds it is the longest path: a ray that grazes
 // the 262K scene's height field walks hundreds of nodes, one dependent read after another. So a tail of at
-// most P.group_tail paths goes to k_tail_group, eight lanes per path over an 8-wide tree; a larger one to
+// most P.group_tail paths goes to k_tail_group, eight lanes per path that visit a treelet at once; a larger one to
 // k_tail, a thread per path.
 template <bool Count, bool Packed>
 __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ WfParams P) {
@@ -1358,19 +1356,20 @@ __global__ void __launch_bounds__(256) k_tail(const __grid_constant__ WfParams P
 // A group of eight lanes per path, four paths per warp in lockstep: the groups' rays are walked together
 // (group_walk.cuh) and their vertices shaded together, each lane of a group computing the same. Bound by the
 // longest path up to some 8,000 paths (the groups in flight), then by issue, which is why larger tails go
-// to k_tail. Frames of the 262K terrain, depth 8, a thread per path -> groups: 4,096 paths 0.97 -> 0.36 ms,
-// 14,400 1.03 -> 0.49, 57,600 1.12 -> 1.2 (not taken); the 36-triangle box, whose rays are short: 4,096
-// paths 0.23 -> 0.20, 16,384 0.27 -> 0.28. (Groups that step on their own, each with the warp masks of its
-// own lanes, run one after another: 14,400 paths 0.56. Leaving a thread's path to the groups after 128 to
-// 512 walk steps: 57,600 paths 1.05-1.2 ms, 115,200 1.24-1.6 against 1.17: not kept.)
+// to k_tail. Frames of the 262K terrain, depth 8, a thread per path -> groups: 4,096 paths 0.97 -> 0.40 ms,
+// 14,400 0.92 -> 0.52, 57,600 slower (not taken); the 36-triangle box, whose rays are short, 16,384 paths:
+// 0.27 -> 0.33 (kSmallTree). Photon's order costs about 12% of that against a walk that takes the nearest child
+// first (14,400 paths: 0.46), whose answers are not always Photon's. (Groups that step on their own, each with
+// the warp masks of its own lanes, run one after another: 0.56 where lockstep took 0.49. Leaving a thread's path
+// to the groups after 128 to 512 walk steps was slower too.)
 __global__ void __launch_bounds__(128) k_tail_group(const __grid_constant__ WfParams P) {
     Counters* c = P.ctr;
     if (!c->tail) return;
     const uint32_t p = c->parity, n = c->count[p];
     if (n > P.group_tail) return;
-    __shared__ uint2 s_stack[128 / kWide][kGroupStack];
-    uint2* stack = s_stack[threadIdx.x / kWide];
-    const uint32_t gl = threadIdx.x & (kWide - 1);
+    __shared__ uint4 s_stack[128 / kTreelet][kGroupStack];
+    uint4* stack = s_stack[threadIdx.x / kTreelet];
+    const uint32_t gl = threadIdx.x & (kTreelet - 1);
     uint32_t rays = 0, shadow_rays = 0;
     PathState st{};
     const DevScene* s = P.scenes;
@@ -1379,7 +1378,7 @@ __global__ void __launch_bounds__(128) k_tail_group(const __grid_constant__ WfPa
         // Each group without a path claims one.
         uint32_t k = n;
         if (!has && !drained && gl == 0) k = atomicAdd(&c->fetch[5], 1u);
-        k = __shfl_sync(kFull, k, 0, kWide);
+        k = __shfl_sync(kFull, k, 0, kTreelet);
         if (!has) {
             drained = k >= n;
             if (!drained) {

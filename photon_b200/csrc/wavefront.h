@@ -145,7 +145,7 @@ cudaError_t wf_iteration(const WfParams& p, const LaunchShape& ls, cudaStream_t 
 constexpr uint32_t kSortMinPaths = 1u << 21;
 // Renders of fewer paths are not shaded in class order over the whole queue.
 constexpr uint32_t kOrderMinPaths = 1u << 18;
-constexpr uint32_t kGroupTail = 1u << 14;  // WfParams::group_tail where every scene has the 8-wide tree
+constexpr uint32_t kGroupTail = 1u << 14;  // WfParams::group_tail where every scene is in treelet order
 // Kernels wf_iteration launches for these parameters.
 inline int wf_kernels_per_iteration(const WfParams& p) {
     return 5 + (p.order ? 3 : 0) + (p.tail_paths > 0 ? (p.group_tail ? 2 : 1) : 0) + (p.sort_bits > 0 ? 3 : 0) + (p.shadow_sort_bits > 0 ? 2 : 0);

@@ -29,6 +29,19 @@ def test_a_path_pool_holds_what_is_counted(cuda):
     assert held <= counted + SLACK
 
 
+def test_a_scene_holds_what_is_counted(cuda):
+    box, g = native.box_scene(), native.terrain_scene(1 << 20, 2)
+    small, b = box.build(), g.build(gpu=True)
+    s = native.Server(path_capacity=1 << 20, reserve_bytes=-1)
+    s.add_scene(small.desc)
+    before, counted = _free(cuda), s.stats().device_bytes_in_use
+    s.add_scene(b.desc)
+    held, counted = before - _free(cuda), s.stats().device_bytes_in_use - counted
+    s.close()
+    assert counted > 150 << 20
+    assert held <= counted + SLACK
+
+
 @pytest.mark.parametrize("kind", ["box", "terrain"])
 def test_the_class_order_beside_sorted_shadow_rays(kind):
     """The order of the shading and that of the shadow walk share their memory: an iteration that has both."""
