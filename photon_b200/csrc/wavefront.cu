@@ -478,9 +478,10 @@ __device__ __forceinline__ void walk_queue_pairs4(uint32_t n, uint32_t* claim, u
 //   another triangle with a distance between t and T's box entry (which rounding can put a little beyond
 //   t), or exactly t, was accepted first. This walk visits nodes in Photon's order and prunes later than
 //   Photon does, at (1 + 2^-10) of the least distance so far, so it tests every triangle that Photon tests
-//   and every such other one. If the second least distance it accepted is within 1 + 2^-14 of the least,
-//   or it accepted a triangle clearly ahead of its own box (one seen edge-on, whose distance is rounding),
-//   the ray is walked again in Photon's order: about one ray in 10,000.
+//   and every such other one. (Photon tests the boxes of a node's two leaves before either's triangles: the
+//   second is not pruned for what the first has.) If the second least distance it accepted is within 1 + 2^-14
+//   of the least, or it accepted a triangle clearly ahead of its own box (one seen edge-on, whose distance is
+//   rounding), the ray is walked again in Photon's order: about one ray in 10,000.
 constexpr uint32_t kListCap = 128;  // entries of a warp's ring; a round of visits appends up to 64
 constexpr int kListStack = 12;      // stack entries per thread kept in shared memory (16: trace +0.5%)
 constexpr uint32_t kListVisits = 2; // rounds per step, per node visit of a pair walk's step (see walk_queue_list)
@@ -497,7 +498,8 @@ struct ListSlots {
     unsigned long long best[AnyHit ? 1 : 32];  // least accepted distance: its bits << 32 | triangle; ~0 none
     const DevScene* scene[Single ? 1 : 32];
     float2 uv[AnyHit ? 1 : 32];                // barycentrics of `best`
-    uint2 list[kListCap];                      // a leaf: (2 * node + side) << 5 | owner's lane, its box entry
+    uint2 list[kListCap];                      // a leaf: (2 * node + side) << 5 | owner's lane; its box entry,
+                                               // negative (-0 too) for the second leaf of a node (closest hit)
     uint8_t start[32];                         // a test round's leaves by their first pair
     uint32_t mark[32];                         // any-hit: 1 once answered; closest: second least distance's bits
 };
@@ -557,7 +559,8 @@ __device__ __forceinline__ void list_test(ListSlots<AnyHit, Single>& ls, bool on
 }
 
 // Tests m listed leaves (at most 32, one per lane) from list position `head` on, 32 pairs at a time; a
-// leaf entered beyond its owner's present limit is dropped.
+// leaf entered beyond its owner's present limit is dropped, but for the second leaf of a node, since the first
+// one's triangles, tested in an earlier call, may have lowered that limit.
 template <bool AnyHit, bool Single>
 __device__ __forceinline__ void list_leaves(ListSlots<AnyHit, Single>& ls, uint32_t head, uint32_t m, const WalkScene& uniform) {
     const uint32_t lane = lane_id(), upto = 0xffffffffu >> (31u - lane);
@@ -567,8 +570,8 @@ __device__ __forceinline__ void list_leaves(ListSlots<AnyHit, Single>& ls, uint3
     if (lane < m) {
         const uint2 e = ls.list[(head + lane) & (kListCap - 1)];
         owner = e.x & 31u;
-        entry = __uint_as_float(e.y);
-        if (entry <= ls.d[owner].w) {
+        entry = fabsf(__uint_as_float(e.y));
+        if (entry <= ls.d[owner].w || (!AnyHit && int(e.y) < 0)) {
             const float4* np = (Single ? uniform.nodes : ls.scene[owner]->nodes) + 2 * size_t(e.x >> 5);
             first = __float_as_int(__ldg(np).w);
             count = uint32_t(__float_as_int(__ldg(np + 1).w));
@@ -686,7 +689,7 @@ __device__ __forceinline__ void walk_queue_list(uint32_t n, uint32_t* claim, uin
                     last = p0 + 1;
                 }
                 if (leaf1) {
-                    ls.list[p1 & (kListCap - 1)] = make_uint2(at | 32u, __float_as_uint(t1));
+                    ls.list[p1 & (kListCap - 1)] = make_uint2(at | 32u, __float_as_uint(!AnyHit && leaf0 ? -t1 : t1));
                     last = p1 + 1;
                 }
                 tail += n0 + uint32_t(__popc(l1));

@@ -10,6 +10,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
+from oracle import oracle as O
 from photon_b200 import abi, native, workloads
 
 pytestmark = pytest.mark.gpu
@@ -148,6 +149,36 @@ def _shifted(kind, tiles=1500):
 
 SCENES = {"fan, pairs": lambda: _fan("pairs"), "fan, apart": lambda: _fan("apart"), "fan, tilted": lambda: _fan("apart", 1e-7),
           "shifted, pairs": lambda: _shifted("pairs"), "shifted, apart": lambda: _shifted("apart")}
+
+
+def _ahead(name, hits):
+    """How many rays end on a triangle ahead of its box."""
+    tri = O.hits_tri(hits)
+    if "shifted" in name:
+        return int(((tri >= 0) & (np.abs(hits[..., 0]) < 1.2) & (tri < 3000)).sum())
+    return int(((tri >= 0) & (tri % 2 == 0 if "pairs" in name else tri < PLANES)).sum())
+
+
+@pytest.mark.parametrize("name", SCENES)
+def test_list_walk_ends_on_photons_hit(name):
+    desc, keep, camera = SCENES[name]()
+    r = native.Renderer()
+    r.upload(desc)
+    assert r.scene_walks()[0] == 1
+    cam = camera(1.28)
+    r.set_tuning(pair_walk=0)
+    want, ahead = r.trace_primary(cam, 96, 75, 0, 1), 0
+    assert np.array_equal(want.view(np.uint32), O.orc_trace_primary(desc, cam, 96, 75, 0, 1).view(np.uint32))
+    for seed in range(2 if "shifted" in name else 12):
+        r.set_tuning(pair_walk=0)
+        want = r.trace_primary(cam, 512, 400, 0, seed)
+        ahead += _ahead(name, want)
+        for visits in (1, 3, 5):
+            r.set_tuning(pair_walk=visits)
+            got = r.trace_primary(cam, 512, 400, 0, seed)
+            assert np.array_equal(got.view(np.uint32), want.view(np.uint32)), (seed, visits)
+    r.close()
+    assert ahead > (300000 if "shifted" in name else 20)
 
 
 @pytest.mark.parametrize("name", SCENES)
