@@ -29,9 +29,10 @@ constexpr int kTailShared = 1 << 16;
 // frames, frames/s with 131,072 (alone) or 65,536 / 16,384 / 8,192 / 4,096: one session 399 / 436 / 401 /
 // 376, two 599 / 600 / 598 / 580, four 699 / 703 / 766 / 770, eight 706 / 704 / 803 / 851.
 constexpr int kGroupTailAlone = 1 << 14;
-constexpr int kGroupTailFew = 1 << 13;   // one or two other renders; or a tree of fewer than kSmallTree nodes (the
-                                         // 36-triangle box, 16,384 paths: 0.28 ms with 16,384, 0.26 with 8,192)
-constexpr int kSmallTree = 512;
+constexpr int kGroupTailFew = 1 << 13;   // one or two other renders; or a tree of fewer than kSmallTree nodes
+// Frames of 16,384 paths, ms with 16,384 / 8,192, over trees of 19 nodes: 0.33 / 0.29, 138: 0.33 / 0.26,
+// 268: 0.38 / 0.30, 541: 0.41 / 0.35; 1,072: 0.28 / 0.30, 2,150: 0.35 / 0.37, 16,859: 0.56 / 0.57.
+constexpr int kSmallTree = 1024;
 constexpr int kGroupTailMany = 1 << 12;
 
 // Tunable launch parameters (the autotuner's knobs).
