@@ -3,7 +3,7 @@
 Device code: nvcc for sm_100a only, with -fmad=false and IEEE division / square root so that the
 integrator's arithmetic rounds like the host reference (see csrc/pt_math.cuh). Host code: g++
 -std=c++20 -O3 for baseline x86-64 (no FMA contraction either). Incremental: an object is rebuilt
-when its source or any header in csrc/ or include/ is newer.
+when its source, any header in csrc/ or include/ or this file is newer.
 
     python -m photon_b200.build [--force] [-j N]
 """
@@ -26,14 +26,11 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-fmad=false", "-prec-div=true", "-prec-sqrt=true",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-O3", *GENCODE]
-# The denoiser's weights are approximate functions whose denormal handling costs as much as they do; it
-# flushes denormals, as Photon's own build of svgf.cu (--use_fast_math) does.
-FILE_FLAGS = {"svgf.cu": ["-ftz=true"]}
 CXX_FLAGS = ["-std=c++20", "-O3", "-fPIC", "-pthread", "-Wall", "-Wno-missing-field-initializers"]
 
 
 def _headers():
-    hs = []
+    hs = [os.path.abspath(__file__)]  # (the flags are here)
     for d in (CSRC, INCLUDE):
         for f in os.listdir(d):
             if f.endswith((".h", ".cuh", ".hpp")):
@@ -51,7 +48,7 @@ def _stale(obj, src, headers):
 def _compile(src, obj):
     inc = ["-I", INCLUDE, "-I", CSRC]
     if src.endswith(".cu"):
-        cmd = [NVCC, *NVCC_FLAGS, *FILE_FLAGS.get(os.path.basename(src), []), *inc, "-c", src, "-o", obj]
+        cmd = [NVCC, *NVCC_FLAGS, *inc, "-c", src, "-o", obj]
     else:
         cxx = shutil.which("g++") or "g++"
         cmd = [cxx, *CXX_FLAGS, *inc, "-I", os.path.join(CUDA_HOME, "include"), "-c", src, "-o", obj]
