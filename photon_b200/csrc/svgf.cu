@@ -167,45 +167,29 @@ __global__ void __launch_bounds__(128) k_temporal(Frame5 in5, SvgfFrame in, Prev
 // history is shorter than 4 frames. The edge-stopping weights use the fast exp / pow that Photon's
 // build (--use_fast_math) gives svgf.cu. A block whose pixels need the estimate stages its pixels and a
 // border of three in shared memory with their directions prepared, once per staged pixel instead of once
-// per tap. With two pixels per thread (Px), one above the other, whose windows share six of eight rows, fewer
-// shared-memory reads bound it (85% of their peak with one). 1600x900, every pixel a surface: 155 us (global
-// loads, directions per tap) -> 98 (staged) -> 83 (two pixels); 427x241, whose 224 blocks of two-pixel threads
-// do not fill the chip: 22.6 -> 13.6 with one, 17.1 with two. So frames below kVarPairs pixels take one.
-constexpr int kVarW = 32, kVarRows = 8, kVarR = 3;  // a block's threads, the window's radius
-constexpr int kVarPairs = 400000;
-template <int Px>
-__global__ void __launch_bounds__(kVarW* kVarRows) k_variance(const float4* __restrict__ edge, int w, int h, const float4* __restrict__ illum,
-                                                               const float4* __restrict__ moments, float phi_normal,
-                                                               float4* __restrict__ out) {
-    constexpr int kVarH = kVarRows * Px, kTw = kVarW + 2 * kVarR, kTh = kVarH + 2 * kVarR;
+// per tap; bound by the shared-memory reads (85% of their peak). One
+// surface all over, 1600x900: 200 us (global loads, directions per tap) -> 125; 427x241: 24.8 -> 15.1. (Two pixels
+// per thread, whose windows share six of eight rows: the same from 500,000 pixels on, slower below.)
+constexpr int kVarW = 32, kVarH = 8, kVarR = 3;  // a block's pixels, the window's radius
+__global__ void __launch_bounds__(kVarW* kVarH) k_variance(const float4* __restrict__ edge, int w, int h, const float4* __restrict__ illum,
+                                                           const float4* __restrict__ moments, float phi_normal, float4* __restrict__ out) {
+    constexpr int kTw = kVarW + 2 * kVarR, kTh = kVarH + 2 * kVarR;
     __shared__ float4 t_dir[kTh * kTw], t_zm[kTh * kTw], t_col[kTh * kTw];  // direction; depth, material, moments; colour
-    const int tx = threadIdx.x, ty = Px * int(threadIdx.y), x = blockIdx.x * kVarW + tx, y = blockIdx.y * kVarH + ty;
-    V3 c[Px], n[Px];
-    float variance[Px], len[Px], z[Px], inv_dz[Px];
-    int mat[Px];
-    bool estimate[Px], some = false;
-#pragma unroll
-    for (int k = 0; k < Px; k++) {
-        const bool on = x < w && y + k < h;
-        float4 cc = make_float4(0, 0, 0, 0), e = cc;
-        variance[k] = 0;
-        if (on) {
-            const int i = (y + k) * w + x;
-            cc = __ldg(illum + i);
-            variance[k] = __ldg(moments + i).z;
-            e = __ldg(edge + i);
-        }
-        c[k] = xyz(cc);
-        len[k] = cc.w;
-        mat[k] = edge_material(e);
-        estimate[k] = on && len[k] < 4.0f && mat[k] >= 0;
-        some = some || estimate[k];
-        n[k] = oct_decode(e.x, e.y);
-        z[k] = e.z;
-        inv_dz[k] = __fdividef(1.0f, 0.05f * e.z + 1e-3f);
+    const int tx = threadIdx.x, ty = threadIdx.y, x = blockIdx.x * kVarW + tx, y = blockIdx.y * kVarH + ty, i = y * w + x;
+    const bool on = x < w && y < h;
+    float4 cc = make_float4(0, 0, 0, 0), e = cc;
+    float variance = 0;
+    if (on) {
+        cc = __ldg(illum + i);
+        variance = __ldg(moments + i).z;
+        e = __ldg(edge + i);
     }
-    if (__syncthreads_or(some)) {
-        for (int k = int(threadIdx.y) * kVarW + tx; k < kTw * kTh; k += kVarW * kVarRows) {
+    V3 c = xyz(cc);
+    const float len = cc.w;
+    const int mat = edge_material(e);
+    const bool estimate = on && len < 4.0f && mat >= 0;
+    if (__syncthreads_or(estimate)) {
+        for (int k = ty * kVarW + tx; k < kTw * kTh; k += kVarW * kVarH) {
             const int xx = int(blockIdx.x) * kVarW + k % kTw - kVarR, yy = int(blockIdx.y) * kVarH + k / kTw - kVarR;
             float4 dir = make_float4(0, 0, 0, 0), zm = make_float4(0, __int_as_float(-1), 0, 0), col = dir;  // (no pixel: no surface)
             if (xx >= 0 && yy >= 0 && xx < w && yy < h) {
@@ -221,37 +205,31 @@ __global__ void __launch_bounds__(kVarW* kVarRows) k_variance(const float4* __re
         }
         __syncthreads();
     }
-    if (some) {
-        float wsum[Px] = {}, m1[Px] = {}, m2[Px] = {};
-        V3 acc[Px] = {};
-        for (int dy = -kVarR; dy < kVarR + Px; dy++)
+    if (estimate) {
+        const V3 n = oct_decode(e.x, e.y);
+        const float z = e.z, inv_dz = __fdividef(1.0f, 0.05f * z + 1e-3f);
+        float wsum = 0, m1 = 0, m2 = 0;
+        V3 acc = v3(0);
+        for (int dy = -kVarR; dy <= kVarR; dy++)
 #pragma unroll
             for (int dx = -kVarR; dx <= kVarR; dx++) {
                 const int j = (ty + kVarR + dy) * kTw + tx + kVarR + dx;
-                const float4 zm = t_zm[j], dir = t_dir[j], col = t_col[j];
-                const int m = __float_as_int(zm.y);
-#pragma unroll
-                for (int k = 0; k < Px; k++) {
-                    if (m != mat[k] || dy < k - kVarR || dy > k + kVarR) continue;
-                    float wt = __expf(log_normal_weight(n[k], dir, phi_normal) - fabsf(zm.x - z[k]) * inv_dz[k]);
-                    m1[k] += zm.z * wt;
-                    m2[k] += zm.w * wt;
-                    acc[k] = acc[k] + xyz(col) * wt;
-                    wsum[k] += wt;
-                }
+                const float4 zm = t_zm[j];
+                if (__float_as_int(zm.y) != mat) continue;
+                const float wt = __expf(log_normal_weight(n, t_dir[j], phi_normal) - fabsf(zm.x - z) * inv_dz);
+                m1 += zm.z * wt;
+                m2 += zm.w * wt;
+                acc = acc + xyz(t_col[j]) * wt;
+                wsum += wt;
             }
-#pragma unroll
-        for (int k = 0; k < Px; k++)
-            if (estimate[k] && wsum[k] > 0) {
-                m1[k] /= wsum[k];
-                m2[k] /= wsum[k];
-                variance[k] = fmaxf(0.0f, m2[k] - m1[k] * m1[k]) * (4.0f / len[k]);
-                c[k] = acc[k] / wsum[k];
-            }
+        if (wsum > 0) {
+            m1 /= wsum;
+            m2 /= wsum;
+            variance = fmaxf(0.0f, m2 - m1 * m1) * (4.0f / len);
+            c = acc / wsum;
+        }
     }
-#pragma unroll
-    for (int k = 0; k < Px; k++)
-        if (x < w && y + k < h) out[(y + k) * w + x] = make_float4(c[k].x, c[k].y, c[k].z, variance[k]);
+    if (on) out[i] = make_float4(c.x, c.y, c.z, variance);
 }
 
 struct AtrousEpilogue {
@@ -359,11 +337,10 @@ struct AtrousTile {
 };
 
 // Preparing a record once per staged pixel takes the direction, its reciprocal root and the luminance, 25 of a
-// tap's 70 instructions, out of the 25 taps; the passes are bound by issue (79%). 1600x900, every pixel a
-// surface, per pass of steps 1 / 2 / 4 / 8 / 16: 94 / 89 / 89 / 100 / 101 us -> 73 / 68 / 76 / 73 / 91 (85 /
-// 79 / 83 / 81 / 98 before denormals were flushed). Strided TMA tiles for steps 8 and 16 took 127 and 154.
-// A block without a surface prepares and filters nothing: frames of a viewer, half of them sky, 449 -> 458 per
-// second.
+// tap's 70 instructions, out of the 25 taps; the passes are bound by issue (79%). 1600x900, one surface all
+// over, per pass of steps 1 / 2 / 4 / 8 / 16: 117 / 113 / 113 / 124 / 129 us -> 96 / 92 / 101 / 101 / 116;
+// 427x241: 14.2 / 13.5 / 13.6 / 14.3 / 17.5 -> 12.2 / 11.6 / 12.2 / 14.1 / 15.5. Strided TMA tiles for steps 8 and
+// 16 took a quarter and a half more than the rows. A block without a surface prepares and filters nothing.
 //
 // atrous_kernel's filter (svgf.cu:134-186) at pixel (x, y), entry ci of the tile, whose taps lie sx and sy
 // entries apart in x and y. The 3x3 variances and the depth gradient come through src_w(x, y) and
@@ -638,10 +615,8 @@ void denoise(const Frame5& in5, const SvgfFrame& in, const PrevCamera& pc, int w
     const float4* edge = edge_out;
     k_temporal<FromPhoton><<<grid, block, 0, stream>>>(in5, in, pc, w, h, has_history ? 1 : 0, s.alpha_color, s.alpha_moments, hist,
                                                        edge_out, illum, moments);
-    const int px = w * h >= kVarPairs ? 2 : 1, var_rows = kVarRows * px;
-    const dim3 var_grid((w + kVarW - 1) / kVarW, (h + var_rows - 1) / var_rows), var_block(kVarW, kVarRows);
-    if (px == 2) k_variance<2><<<var_grid, var_block, 0, stream>>>(edge, w, h, illum, moments, s.phi_normal, f0);
-    else k_variance<1><<<var_grid, var_block, 0, stream>>>(edge, w, h, illum, moments, s.phi_normal, f0);
+    k_variance<<<dim3((w + kVarW - 1) / kVarW, (h + kVarH - 1) / kVarH), dim3(kVarW, kVarH), 0, stream>>>(edge, w, h, illum, moments,
+                                                                                                          s.phi_normal, f0);
     AtrousEpilogue last{};
     last.output = reinterpret_cast<float4*>(output);
     last.color = FromPhoton ? in5.color : in.color;
