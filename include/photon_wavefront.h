@@ -378,16 +378,16 @@ int32_t pt_svgf_reset(pt_svgf* s);
 int32_t pt_svgf_run(pt_svgf* s, const float* color, const float* albedo, const float* normal_depth,
                     const float* position, const float* emission, const pt_camera* previous,
                     const pt_svgf_settings* settings, float* output);
-/* The variance estimate of the last run (Svgf::variance_buffer, svgf.h:44): a device pointer. */
-/* How the a-trous passes read their 5x5 taps. Without this call: from shared-memory tiles that the Tensor
- * Memory Accelerator stages for steps 1-4, and rows staged by plain loads for steps 8 and 16. 0: from
- * global memory; 1: contiguous tiles for steps 1-8 and global loads beyond; 2 as 1 plus a strided tile (one residue class of x, y mod 8) for step 16; 3 strided tiles
- * for steps 1-16. Every mode gives the same output bit for bit. */
+/* How the a-trous passes read their 5x5 taps. 0: from global memory; 1: from contiguous shared-memory tiles that
+ * the Tensor Memory Accelerator stages for steps 1-8, global loads beyond; 2: as 1 with a strided tile (one residue
+ * class of x, y mod 8) for step 16; 3: strided tiles for steps 1-16; 4 (default): contiguous tiles for steps 1-4,
+ * rows staged by plain loads for steps 8 and 16, global loads beyond. Every mode gives the same output bit for bit. */
 int32_t pt_svgf_set_tma(pt_svgf* s, int32_t mode);
 /* Test hook for the TMA passes' bounded wait (no counterpart in Photon): with on = 1 they arm their
  * tile barrier without issuing the tile copies and wait 2 us, so the wait runs out with no copy in
  * flight; the timeout is reported as PT_ERR_CUDA by the next pt_svgf_run, and the frame is invalid. */
 int32_t pt_svgf_debug_tma_timeout(pt_svgf* s, int32_t on);
+/* The variance estimate of the last run (Svgf::variance_buffer, svgf.h:44): a device pointer. */
 const float* pt_svgf_variance(const pt_svgf* s);
 const char* pt_svgf_last_error(const pt_svgf* s);
 

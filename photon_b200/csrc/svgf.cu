@@ -811,7 +811,7 @@ void SvgfDenoiser::build_tma_plan() {
 }
 
 void SvgfDenoiser::set_tma(int mode) {
-    if (mode < 0 || mode > 3) throw Error{PT_ERR_INVALID, "TMA mode must be in [0, 3]"};
+    if (mode < 0 || mode > kTmaDefault) throw Error{PT_ERR_INVALID, "TMA mode must be in [0, 4]"};
     tma_mode_ = mode;
     build_tma_plan();
 }

@@ -19,7 +19,7 @@ struct TmaPass {
 };
 constexpr int kRowsPass = 0;
 
-constexpr int kTmaDefault = 4;  // the staging used unless set_tma chooses one of 0 to 3
+constexpr int kTmaDefault = 4;  // the staging used unless set_tma chooses another
 
 class SvgfDenoiser {
 public:
@@ -29,7 +29,7 @@ public:
     SvgfDenoiser& operator=(const SvgfDenoiser&) = delete;
     void resize(int w, int h);
     // How the a-trous passes stage their taps (pt_svgf_set_tma): 0 global loads; 1-3 TMA-staged
-    // shared-memory tiles for some steps (see tma_passes_for_mode in svgf.cu).
+    // shared-memory tiles for some steps, 4 those and staged rows (see tma_passes_for_mode in svgf.cu).
     void set_tma(int mode);
     bool tma_active() const { return maps_ok_; }
     // Test hook: the TMA passes arm their tile barrier without issuing the copies and wait 2 us, so

@@ -339,7 +339,7 @@ class Svgf:
         lib.pt_svgf_reset(self.h)
 
     def set_tma(self, mode):
-        """0 global loads, 1-3 TMA-staged tiles (pt_svgf_set_tma)."""
+        """0 global loads, 1-3 TMA-staged tiles, 4 (default) tiles and staged rows (pt_svgf_set_tma)."""
         _check(lib.pt_svgf_set_tma(self.h, int(mode)), lambda: lib.pt_svgf_last_error(self.h))
 
     def debug_tma_timeout(self, on):
