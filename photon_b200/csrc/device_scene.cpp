@@ -137,6 +137,7 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     validate_scene(d, lights_only);
     if (!lights_only) {
         d_view_.allocate(1);
+        light_work_.release();
         nodes_.upload(reinterpret_cast<const float4*>(d.nodes), size_t(d.num_nodes) * 4, s);
         // The 4-wide BVH for any-hit rays, collapsed from the same tree (absent if it does not fit
         // the walk's stack or leaf encoding; the shadow rays then walk the BVH2).

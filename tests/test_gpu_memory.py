@@ -42,6 +42,22 @@ def test_a_scene_holds_what_is_counted(cuda):
     assert held <= counted + SLACK
 
 
+def test_a_light_rebuild_keeps_little(cuda):
+    """Its scratch is 36 bytes per triangle and 12 per texel, 81 MB here; what stays is at most 32 MiB."""
+    g = native.terrain_scene(1 << 21, 2)
+    b = g.build(gpu=True)
+    raw = g.raw
+    u = abi.LightUpdate(raw.materials, raw.num_materials, raw.punctual, raw.num_punctual, raw.env_texels, raw.env_width,
+                        raw.env_height, raw.env_color, raw.env_intensity, raw.env_rotation)
+    r = native.Renderer()
+    r.upload(b.desc)
+    before = _free(cuda)
+    r.rebuild_lights(u)
+    held = before - _free(cuda)
+    r.close()
+    assert held <= (32 << 20) + SLACK
+
+
 @pytest.mark.parametrize("kind", ["box", "terrain"])
 def test_the_class_order_beside_sorted_shadow_rays(kind):
     """The order of the shading and that of the shadow walk share their memory: an iteration that has both."""
