@@ -50,7 +50,7 @@ WavefrontEngine::WavefrontEngine(int device, cudaStream_t stream) : device_(devi
 }
 
 WavefrontEngine::~WavefrontEngine() {
-    if (graph_) cudaGraphExecDestroy(graph_);
+    drop_graphs();
     for (cudaEvent_t e : prof_ev_) cudaEventDestroy(e);
     if (ev_) cudaEventDestroy(ev_);
     if (h_ctr_) cudaFreeHost(h_ctr_);
@@ -66,20 +66,14 @@ void WavefrontEngine::set_tuning(const Tuning& t) {
         for (auto& b : ids_) b.release();
         pb_ = PathBuffers{};
     }
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
+    drop_graphs();
 }
 
 void WavefrontEngine::set_profiling(int flags) {
     profile_flags_ = flags;
     for (double& m : kernel_ms) m = 0;
     kernel_launches = iteration_launches = 0;
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
+    drop_graphs();
     int need = 6 * std::max(1, tuning_.graph_bounces);
     while (int(prof_ev_.size()) < need) {
         cudaEvent_t e;
@@ -120,17 +114,11 @@ void WavefrontEngine::reserve_paths(uint64_t needed) {
     shadow_keys_.allocate(want);
     shadow_perm_.allocate(want);
     pb_.capacity = uint32_t(want);
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
+    drop_graphs();
 }
 
 void WavefrontEngine::release_paths() {
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
-    }
+    drop_graphs();
     for (auto& b : bufs_) b.release();
     for (auto& b : ids_) b.release();
     for (DeviceBuffer<uint32_t>* b : {&keys_, &hist_, &offsets_, &shadow_keys_, &shadow_hist_, &shadow_offsets_, &shadow_perm_}) b->release();
@@ -211,11 +199,29 @@ WfParams WavefrontEngine::params(const DevScene* scenes, int single, const DevSc
     return p;
 }
 
-void WavefrontEngine::capture(const WfParams& p) {
-    if (graph_) {
-        cudaGraphExecDestroy(graph_);
-        graph_ = nullptr;
+void WavefrontEngine::drop_graphs() {
+    for (Graph& g : graphs_) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
     }
+}
+
+// The captured iterations for these parameters. The last two are kept: a caller that alternates two renders, of
+// which one is shaded in class order or sorted and the other not, captured one anew per render (0.2 ms).
+const WavefrontEngine::Graph& WavefrontEngine::graph_for(const WfParams& p) {
+    for (Graph& g : graphs_) {
+        if (!g.exec || std::memcmp(&g.params, &p, sizeof(p)) != 0 || g.iterations != tuning_.graph_bounces) continue;
+        if (&g != &graphs_[0]) std::swap(graphs_[0], graphs_[1]);
+        return graphs_[0];
+    }
+    std::swap(graphs_[0], graphs_[1]);
+    capture(p, graphs_[0]);
+    return graphs_[0];
+}
+
+void WavefrontEngine::capture(const WfParams& p, Graph& out) {
+    if (out.exec) cudaGraphExecDestroy(out.exec);
+    out.exec = nullptr;
     int iters = std::max(1, tuning_.graph_bounces);
     cudaGraph_t g = nullptr;
     bool timed = (profile_flags_ & PT_PROFILE_KERNEL_TIMES) && int(prof_ev_.size()) >= 6 * iters;
@@ -232,14 +238,14 @@ void WavefrontEngine::capture(const WfParams& p) {
         if (g) cudaGraphDestroy(g);
         throw Error{PT_ERR_CUDA, std::string("graph capture failed: ") + cudaGetErrorString(e)};
     }
-    e = cudaGraphInstantiate(&graph_, g, 0);
+    e = cudaGraphInstantiate(&out.exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
-        graph_ = nullptr;
+        out.exec = nullptr;
         throw Error{PT_ERR_CUDA, std::string("graph instantiation failed: ") + cudaGetErrorString(e)};
     }
-    graph_params_ = p;
-    graph_iters_ = iters;
+    out.params = p;
+    out.iterations = iters;
 }
 
 void WavefrontEngine::run(const DevScene* scenes, int single_scene, const DevScene* single, const DevView* views, int n_views,
@@ -264,12 +270,12 @@ void WavefrontEngine::run(const DevScene* scenes, int single_scene, const DevSce
     if (std::min<uint64_t>(total_work, uint64_t(tuning_.path_capacity)) < kOrderMinPaths) p.order = nullptr;
     bool use_graph = tuning_.graph_bounces > 0;
     bool timed = (profile_flags_ & PT_PROFILE_KERNEL_TIMES) != 0;
-    if (use_graph && (!graph_ || std::memcmp(&graph_params_, &p, sizeof(p)) != 0 || graph_iters_ != tuning_.graph_bounces)) capture(p);
+    const Graph* graph = use_graph ? &graph_for(p) : nullptr;
     const uint64_t max_launches = 1u << 22;
     for (uint64_t launch = 0;; launch++) {
-        int iters = use_graph ? graph_iters_ : 1;
-        if (use_graph) {
-            PTW_CUDA(cudaGraphLaunch(graph_, stream_));
+        int iters = graph ? graph->iterations : 1;
+        if (graph) {
+            PTW_CUDA(cudaGraphLaunch(graph->exec, stream_));
         } else {
             PTW_CUDA(wf_iteration(p, shape_, stream_, timed ? prof_ev_.data() : nullptr));
             PTW_CUDA(cudaMemcpyAsync(h_ctr_, ctr_.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream_));

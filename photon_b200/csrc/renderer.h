@@ -135,7 +135,6 @@ public:
 
 private:
     void ensure_shape();
-    void capture(const WfParams& p);
     WfParams params(const DevScene* scenes, int single, const DevScene* single_host, const DevView* views, int n, bool count) const;
 
     int device_;
@@ -152,9 +151,15 @@ private:
     DeviceBuffer<uint32_t> shadow_keys_, shadow_hist_, shadow_offsets_, shadow_perm_;
     Counters* h_ctr_ = nullptr;
     Counters last_{};
-    cudaGraphExec_t graph_ = nullptr;
-    WfParams graph_params_{};
-    int graph_iters_ = 0;
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        WfParams params{};
+        int iterations = 0;
+    };
+    Graph graphs_[2];  // the last one used, and the one before it
+    const Graph& graph_for(const WfParams& p);
+    void capture(const WfParams& p, Graph& out);
+    void drop_graphs();
     cudaEvent_t ev_ = nullptr;
     // continuous mode
     WfParams cont_params_{};

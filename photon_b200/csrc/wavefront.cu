@@ -15,6 +15,10 @@
 // Kernels are persistent: a grid sized to fill the GPU claims 32-path chunks with one atomic per
 // warp until the iteration's count (read from device memory) is exhausted. Compiled with
 // -fmad=false and IEEE division / square root: see pt_math.cuh.
+#include <array>
+#include <map>
+#include <mutex>
+
 #include "wavefront.h"
 #include "gbuffer.cuh"
 
@@ -1971,11 +1975,16 @@ __global__ void k_display(DisplayParams p, const float4* accum, const float4* de
 
 // A list walk's dynamic shared memory: the block's stacks, then a ListSlots per warp.
 template <bool AnyHit, bool Single>
-static size_t list_smem_bytes(int block) {
+static constexpr size_t list_smem_bytes(int block) {
     return size_t(kListStack) * size_t(block) * sizeof(int) + size_t(block / 32) * sizeof(ListSlots<AnyHit, Single>);
 }
+// No walk asks for more dynamic shared memory than a kernel may have without an attribute. (The attribute is the
+// kernel's, not the renderer's: set to what one block size needs, it would refuse the launches of a larger one.)
+constexpr int kMostTraceBlock = 256;
+static_assert(list_smem_bytes<false, false>(kMostTraceBlock) <= 48 << 10);
+static_assert(size_t(kSmemStack) * kMostTraceBlock * sizeof(int) + kMostTraceBlock / 32 * sizeof(PairSlots) <= 48 << 10);
 
-cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, LaunchShape* out) {
+static cudaError_t find_launch_shape(int device, int trace_block, int shade_block, LaunchShape* out) {
     cudaDeviceProp prop;
     cudaError_t e = cudaGetDeviceProperties(&prop, device);
     if (e != cudaSuccess) return e;
@@ -1987,40 +1996,13 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
     out->gen_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     out->trace_block = trace_block;
     size_t smem = size_t(kSmemStack) * trace_block * sizeof(int);
-#define PTW_TRACE_KERNELS(S) (const void*)k_trace<false, false, S>, (const void*)k_trace<false, true, S>, \
-                             (const void*)k_trace<true, false, S>, (const void*)k_trace<true, true, S>
-#define PTW_SHADOW_KERNELS(W, S) (const void*)k_shadow<false, false, W, S>, (const void*)k_shadow<false, true, W, S>, \
-                                 (const void*)k_shadow<true, false, W, S>, (const void*)k_shadow<true, true, W, S>
-    const void* smem_kernels[] = {PTW_TRACE_KERNELS(false), PTW_TRACE_KERNELS(true), PTW_SHADOW_KERNELS(false, false),
-                                  PTW_SHADOW_KERNELS(false, true), PTW_SHADOW_KERNELS(true, false), PTW_SHADOW_KERNELS(true, true)};
-#undef PTW_TRACE_KERNELS
-#undef PTW_SHADOW_KERNELS
-    for (const void* k : smem_kernels) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return e;
-    }
     const size_t pair_smem = smem + size_t(trace_block / 32) * sizeof(PairSlots);
-    const void* pair_kernels[] = {(const void*)k_trace_pairs<false, false>,         (const void*)k_trace_pairs<false, true>,
-                                  (const void*)k_trace_pairs<true, false>,          (const void*)k_trace_pairs<true, true>,
-                                  (const void*)k_shadow_pairs<false, false, false>, (const void*)k_shadow_pairs<false, true, false>,
-                                  (const void*)k_shadow_pairs<true, false, false>,  (const void*)k_shadow_pairs<true, true, false>,
-                                  (const void*)k_shadow_pairs<false, true, true>,   (const void*)k_shadow_pairs<true, true, true>};
-    for (const void* k : pair_kernels) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(pair_smem));
-        if (e != cudaSuccess) return e;
-    }
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_pairs<false, false>, trace_block, pair_smem);
     if (e != cudaSuccess) return e;
     out->pair_trace_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shadow_pairs<false, false, false>, trace_block, pair_smem);
     if (e != cudaSuccess) return e;
     out->pair_shadow_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
-    const void* list_kernels[] = {(const void*)k_trace_list<false>, (const void*)k_trace_list<true>, (const void*)k_shadow_list<false>,
-                                  (const void*)k_shadow_list<true>};
-    for (const void* k : list_kernels) {
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(list_smem_bytes<false, false>(trace_block)));
-        if (e != cudaSuccess) return e;
-    }
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_list<false>, trace_block, list_smem_bytes<false, false>(trace_block));
     if (e != cudaSuccess) return e;
     out->list_trace_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
@@ -2049,6 +2031,23 @@ cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, Launch
     if (e != cudaSuccess) return e;
     out->misses_grid = prop.multiProcessorCount * (nb > 0 ? nb : 1);
     return cudaSuccess;
+}
+
+// A shape depends on the device's kind and the block sizes alone, and finding one takes a dozen calls: each is found
+// once.
+cudaError_t wf_launch_shape(int device, int trace_block, int shade_block, LaunchShape* out) {
+    static std::mutex mu;
+    static std::map<std::array<int, 3>, LaunchShape> found;
+    const std::array<int, 3> key{device, trace_block, shade_block};
+    std::lock_guard<std::mutex> g(mu);
+    const auto it = found.find(key);
+    if (it != found.end()) {
+        *out = it->second;
+        return cudaSuccess;
+    }
+    const cudaError_t e = find_launch_shape(device, trace_block, shade_block, out);
+    if (e == cudaSuccess) found[key] = *out;
+    return e;
 }
 
 template <bool Count, bool Packed, bool Single>
