@@ -254,12 +254,11 @@ int32_t pt_scene_walks(const pt_renderer* r, int32_t* order_free, int32_t* group
 
 int32_t pt_bvh_levels(const pt_bvh_node* nodes, int32_t num_nodes) {
     if (!nodes || num_nodes < 1) return -1;
-    for (int32_t i = 0; i < num_nodes; i++) {
-        const pt_bvh_node& b = nodes[i];
-        if (b.lcount <= 0 && b.left >= 0 && (b.left <= i || b.left >= num_nodes)) return -1;
-        if (b.rcount <= 0 && b.right >= 0 && (b.right <= i || b.right >= num_nodes)) return -1;
+    try {
+        return bvh_levels(nodes, num_nodes, INT32_MAX);
+    } catch (...) {
+        return -1;
     }
-    return bvh_levels(nodes, num_nodes);
 }
 
 int32_t pt_light_picks_primary(pt_renderer* r, const pt_camera* camera, const pt_render_settings* settings, uint32_t frame, int32_t* picks4) {

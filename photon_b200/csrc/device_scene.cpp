@@ -26,24 +26,38 @@ float lum_host(const pt_vec3& c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722
 
 }  // namespace
 
-void validate_scene(const pt_scene_desc& d, bool lights_only) {
+int bvh_levels(const pt_bvh_node* nodes, int32_t n, int32_t num_tris) {
+    std::vector<uint8_t> level(size_t(n), 0);  // 0: no parent so far
+    int most = 1;
+    bool tree = true;
+    for (int32_t i = 0; i < n; i++) {
+        const pt_bvh_node& b = nodes[i];
+        const int32_t idx[2] = {b.left, b.right}, cnt[2] = {b.lcount, b.rcount};
+        const int next = std::min(std::max<int>(level[size_t(i)], 1) + 1, 255);
+        for (int k = 0; k < 2; k++) {
+            if (cnt[k] > 0) {
+                if (idx[k] < 0 || int64_t(idx[k]) + cnt[k] > num_tris) invalid("leaf range outside the triangles");
+                continue;
+            }
+            if (idx[k] >= n) invalid("child node index out of range");
+            if (idx[k] < 0) continue;
+            if (idx[k] <= i) invalid("child node index does not follow its parent (depth-first order)");
+            uint8_t& l = level[size_t(idx[k])];
+            tree = tree && l == 0;
+            l = uint8_t(next);
+            most = std::max(most, next);
+        }
+    }
+    return tree ? most : 0;
+}
+
+int validate_scene(const pt_scene_desc& d, bool lights_only) {
+    int levels = 0;
     if (d.num_tris < 0 || d.num_nodes < 0 || d.num_vertices < 0 || d.num_materials < 0) invalid("negative count");
     if (!lights_only) {
         if (d.num_nodes < 1 || !d.nodes) invalid("a BVH needs at least its root node");
         if (d.num_tris > 0 && (!d.tris || !d.indices)) invalid("triangles without geometry or indices");
-        for (int32_t i = 0; i < d.num_nodes; i++) {
-            const pt_bvh_node& n = d.nodes[i];
-            const int32_t idx[2] = {n.left, n.right}, cnt[2] = {n.lcount, n.rcount};
-            for (int k = 0; k < 2; k++) {
-                if (cnt[k] > 0) {
-                    if (idx[k] < 0 || int64_t(idx[k]) + cnt[k] > d.num_tris) invalid("leaf range outside the triangles");
-                } else if (idx[k] >= d.num_nodes) {
-                    invalid("child node index out of range");
-                } else if (idx[k] >= 0 && idx[k] <= i) {
-                    invalid("child node index does not follow its parent (depth-first order)");
-                }
-            }
-        }
+        levels = bvh_levels(d.nodes, d.num_nodes, d.num_tris);
         for (int64_t i = 0; i < int64_t(d.num_tris) * 3; i++)
             if (d.indices[i] < 0 || d.indices[i] >= d.num_vertices) invalid("vertex index out of range");
     }
@@ -75,25 +89,7 @@ void validate_scene(const pt_scene_desc& d, bool lights_only) {
     if (d.env_texels) {
         if (d.env_width <= 0 || d.env_height <= 0 || !d.env_marginal || !d.env_conditional) invalid("environment tables missing");
     }
-}
-
-int bvh_levels(const pt_bvh_node* nodes, int32_t n) {
-    std::vector<uint8_t> level(size_t(n), 0);  // 0: no parent so far
-    level[0] = 1;
-    int most = 1;
-    for (int32_t i = 0; i < n; i++) {
-        const pt_bvh_node& b = nodes[i];
-        const int32_t idx[2] = {b.left, b.right}, cnt[2] = {b.lcount, b.rcount};
-        const int next = std::min(std::max<int>(level[size_t(i)], 1) + 1, 255);
-        for (int k = 0; k < 2; k++) {
-            if (cnt[k] > 0 || idx[k] < 0) continue;
-            uint8_t& l = level[size_t(idx[k])];
-            if (l) return 0;
-            l = uint8_t(next);
-            most = std::max(most, next);
-        }
-    }
-    return most;
+    return levels;
 }
 
 size_t DeviceScene::estimate_bytes(const pt_scene_desc& d) {
@@ -131,14 +127,44 @@ void DeviceScene::upload_shade_keys(const pt_material* materials, int32_t n, cud
     PTW_CUDA(cudaStreamSynchronize(s));
 }
 
+// The BVH2's nodes, in treelet order for the tail by groups of lanes if the tree is one that it can take. The nodes
+// as they come wait in the triangles' memory, with the scratch in that of the vertex indices, both filled later.
+void DeviceScene::upload_nodes(const pt_scene_desc& d, cudaStream_t s) {
+    const float4* src = reinterpret_cast<const float4*>(d.nodes);
+    const size_t n = size_t(d.num_nodes);
+    int* const root_size = reinterpret_cast<int*>(d_view_.ptr);
+    in_treelets_ = tree_levels_ > 0 && tree_levels_ <= kOrderFreeDepth;
+    DeviceBuffer<float4> own_raw;
+    DeviceBuffer<int> own_work;
+    float4* raw = nullptr;
+    int* work = nullptr;
+    if (in_treelets_ && d.num_nodes > kTreeletBlock) {
+        if (d.num_nodes < d.num_tris) {
+            static_assert(kTriStride == 4 && sizeof(int4) == 4 * sizeof(int), "a triangle's room holds a node's");
+            tris_.allocate(size_t(d.num_tris) * kTriStride);
+            tri_idx_.allocate(size_t(d.num_tris));
+            raw = tris_.ptr;
+            work = reinterpret_cast<int*>(tri_idx_.ptr);
+        } else if ((in_treelets_ = own_raw.try_allocate(4 * n) && own_work.try_allocate(treelet_work(d.num_nodes)))) {
+            raw = own_raw.ptr;  // (more nodes than triangles: a hand-made tree)
+            work = own_work.ptr;
+        }
+    }
+    nodes_.allocate(4 * n);
+    if (!raw) raw = nodes_.ptr;
+    PTW_CUDA(cudaMemcpyAsync(raw, src, n * sizeof(pt_bvh_node), cudaMemcpyHostToDevice, s));
+    if (in_treelets_) order_by_treelets(raw, nodes_.ptr, work, d.num_nodes, tree_levels_, root_size, s);
+}
+
 void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_only) {
     if (lights_only && !ready_) lights_only = false;
     if (lights_only && d.num_tris != view_.num_tris) throw Error{PT_ERR_INVALID, "update_lights: the triangle count changed"};
-    validate_scene(d, lights_only);
+    const int levels = validate_scene(d, lights_only);
     if (!lights_only) {
         d_view_.allocate(1);
         light_work_.release();
-        nodes_.upload(reinterpret_cast<const float4*>(d.nodes), size_t(d.num_nodes) * 4, s);
+        tree_levels_ = levels;
+        upload_nodes(d, s);
         // The 4-wide BVH for any-hit rays, collapsed from the same tree (absent if it does not fit
         // the walk's stack or leaf encoding; the shadow rays then walk the BVH2).
         std::vector<Bvh4Node> wide;
@@ -149,11 +175,6 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
         } else {
             nodes4_.release();
         }
-        // In treelet order for the tail by groups of lanes, before the other arrays take memory: the copy that
-        // this needs for a moment is no more than they will.
-        tree_levels_ = bvh_levels(d.nodes, d.num_nodes);
-        const bool shallow = tree_levels_ > 0 && tree_levels_ <= kOrderFreeDepth;
-        root_treelet_ = shallow ? order_by_treelets(nodes_, d.num_nodes, tree_levels_, reinterpret_cast<int*>(d_view_.ptr), s) : 0;
         num_vertices_ = d.num_vertices;
         if (d.normals) {
             std::vector<float4> n(size_t(d.num_vertices));
@@ -263,7 +284,13 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     v.p_punctual = d.p_punctual;
     v.has_lights = (d.p_env + d.p_emissive + d.p_punctual) > 0 ? 1 : 0;
     v.bvh_depth = tree_levels_;
-    v.order_free = tree_is_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_levels_, reinterpret_cast<int*>(d_view_.ptr), s) ? 1 : 0;
+    int* const found = reinterpret_cast<int*>(d_view_.ptr);  // the root treelet's size, the check's result
+    const bool checked = check_order_free(nodes_.ptr, v.num_nodes, tris_.ptr, tree_levels_, found + 1, s);
+    int h[2] = {0, 1};
+    PTW_CUDA(cudaMemcpyAsync(h, found, sizeof(h), cudaMemcpyDeviceToHost, s));
+    PTW_CUDA(cudaStreamSynchronize(s));
+    if (!lights_only) root_treelet_ = in_treelets_ ? h[0] : 0;
+    v.order_free = checked && h[1] == 0 ? 1 : 0;
     v.root_treelet = v.order_free ? root_treelet_ : 0;
     {
         float lo[3] = {d.bounds_min.x, d.bounds_min.y, d.bounds_min.z}, hi[3] = {d.bounds_max.x, d.bounds_max.y, d.bounds_max.z};

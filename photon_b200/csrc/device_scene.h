@@ -119,17 +119,20 @@ private:
     int32_t num_vertices_ = 0;
     int32_t num_materials_ = 0;
     int tree_levels_ = 0;   // bvh_levels of the uploaded tree
-    int root_treelet_ = 0;  // order_by_treelets of it, 0 if it keeps the order it came in
+    bool in_treelets_ = false;
+    int root_treelet_ = 0;  // the size of its root's treelet, 0 if it keeps the order it came in
+    void upload_nodes(const pt_scene_desc& d, cudaStream_t s);
     void upload_shade_keys(const pt_material* materials, int32_t n, cudaStream_t s);
     float bounds_[6] = {0, 0, 0, 0, 0, 0};  // the scene box (lo xyz, hi xyz), for the light-group weights
 };
 
-// Checks a scene description for internal consistency; throws Error(PT_ERR_INVALID).
-void validate_scene(const pt_scene_desc& d, bool lights_only);
+// Checks a scene description for internal consistency; throws Error(PT_ERR_INVALID). Returns bvh_levels of its tree
+// (0 with lights_only).
+int validate_scene(const pt_scene_desc& d, bool lights_only);
 
-// The levels of a BVH whose children follow their parents (255 and more: 255), or 0 where two parents name
-// one node, which validate_scene lets through: the walks in Photon's order take such a graph as it is, but
-// what counts on a tree's depth or on its number of nodes does not.
-int bvh_levels(const pt_bvh_node* nodes, int32_t n);
+// The levels of a BVH (255 and more: 255), or 0 where two parents name one node, which is let through: the walks in
+// Photon's order take such a graph as it is, but what counts on a tree's depth or on its number of nodes does not.
+// Throws Error(PT_ERR_INVALID) where a child does not follow its parent or an index is out of range.
+int bvh_levels(const pt_bvh_node* nodes, int32_t n, int32_t num_tris);
 
 }  // namespace ptw

@@ -48,7 +48,7 @@ struct DevScene {
     float p_env, p_emissive, p_punctual;
     int has_lights;
     int bvh_depth;
-    int order_free;    // 1: the tree may be walked out of order (tree_is_order_free)
+    int order_free;    // 1: the tree may be walked out of order (check_order_free)
     int root_treelet;  // > 0: order_free, with its nodes in treelet order; the size of the root's treelet
     float bounds_lo_x, bounds_lo_y, bounds_lo_z;   // scene box (for ray-sort keys)
     float inv_extent_x, inv_extent_y, inv_extent_z;

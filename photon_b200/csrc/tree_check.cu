@@ -53,16 +53,13 @@ __global__ void __launch_bounds__(256) k_check_tree(const float4* __restrict__ n
 
 }  // namespace
 
-bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, int* word, cudaStream_t stream) {
+bool check_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, int* bad, cudaStream_t stream) {
     // A list entry keeps 2 * node + side in 27 bits.
     if (levels < 1 || levels > kOrderFreeDepth || num_nodes < 1 || num_nodes >= (1 << 26)) return false;
-    PTW_CUDA(cudaMemsetAsync(word, 0, sizeof(int), stream));
-    k_check_tree<<<(2 * num_nodes + 255) / 256, 256, 0, stream>>>(nodes, num_nodes, tris, word);
+    PTW_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), stream));
+    k_check_tree<<<(2 * num_nodes + 255) / 256, 256, 0, stream>>>(nodes, num_nodes, tris, bad);
     PTW_CUDA(cudaGetLastError());
-    int h = 1;
-    PTW_CUDA(cudaMemcpyAsync(&h, word, sizeof(h), cudaMemcpyDeviceToHost, stream));
-    PTW_CUDA(cudaStreamSynchronize(stream));
-    return h == 0;
+    return true;
 }
 
 }  // namespace ptw

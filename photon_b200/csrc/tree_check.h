@@ -7,10 +7,10 @@ namespace ptw {
 
 constexpr int kOrderFreeDepth = 60;  // levels of the tree: Photon's 64-entry stack then never drops a node
 
-// True when every box of the device-resident tree is finite, ordered and inside its parent's, every leaf's
-// triangles lie inside its box (to rounding), no node has two parents and the tree is at most kOrderFreeDepth
-// levels deep (`levels`: bvh_levels of it), and its nodes fit the list walk's entries. `word`: an int of device
-// scratch. Synchronises the stream.
-bool tree_is_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, int* word, cudaStream_t stream);
+// Whether every box of the device-resident tree is finite, ordered and inside its parent's and every leaf's triangles
+// lie inside its box (to rounding): *bad, on the device and in stream order, becomes 0 then and 1 otherwise. False, with
+// nothing done, where a node has two parents, the tree is more than kOrderFreeDepth levels deep (`levels`: bvh_levels of
+// it) or its nodes do not fit the list walk's entries.
+bool check_order_free(const float4* nodes, int num_nodes, const float4* tris, int levels, int* bad, cudaStream_t stream);
 
 }  // namespace ptw

@@ -12,8 +12,6 @@ namespace ptw {
 
 namespace {
 
-constexpr int kBlockTree = 512;  // nodes of a tree that one block orders in its shared memory
-
 struct Side {
     float4 lo, hi;  // with the index and the count
     __device__ int index() const { return __float_as_int(lo.w); }
@@ -102,9 +100,14 @@ __device__ void write_treelet(const float4* nodes, float4* out, const Places& p,
     }
 }
 
-__global__ void k_next_level(Levels* st) {
-    st->begin = st->end;
-    st->end = st->treelets;
+__global__ void k_next_level(Places p, Levels* st, bool first) {
+    if (first) {
+        p.root[0] = 0;
+        *st = Levels{0, 1, 1, 0};
+    } else {
+        st->begin = st->end;
+        st->end = st->treelets;
+    }
 }
 
 __global__ void __launch_bounds__(128) k_choose(const float4* __restrict__ nodes, Places p, Levels* st) {
@@ -112,15 +115,17 @@ __global__ void __launch_bounds__(128) k_choose(const float4* __restrict__ nodes
     for (int t = st->begin + int(blockIdx.x * blockDim.x + threadIdx.x); t < st->end; t += step) choose_treelet(nodes, p, st, t);
 }
 
-__global__ void __launch_bounds__(128) k_write(const float4* __restrict__ nodes, float4* __restrict__ out, Places p, const Levels* st) {
+__global__ void __launch_bounds__(128) k_write(const float4* __restrict__ nodes, float4* __restrict__ out, Places p, const Levels* st,
+                                                int* __restrict__ root_size) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *root_size = p.size[0];
     const int step = int(gridDim.x * blockDim.x);
     for (int t = int(blockIdx.x * blockDim.x + threadIdx.x); t < st->treelets; t += step) write_treelet(nodes, out, p, t);
 }
 
-// A tree of at most kBlockTree nodes, in place, by one block: no scratch, no allocation, one launch.
-__global__ void __launch_bounds__(128) k_order_block(float4* __restrict__ nodes, int n, int* __restrict__ root_size) {
-    __shared__ float4 s_nodes[4 * kBlockTree];
-    __shared__ int s_places[4][kBlockTree];
+// A small tree, by one block in its shared memory (nodes may be ordered).
+__global__ void __launch_bounds__(128) k_order_block(const float4* nodes, float4* ordered, int n, int* root_size) {
+    __shared__ float4 s_nodes[4 * kTreeletBlock];
+    __shared__ int s_places[4][kTreeletBlock];
     __shared__ Levels st;
     const Places p{s_places[0], s_places[1], s_places[2], s_places[3]};
     for (int k = threadIdx.x; k < 4 * n; k += blockDim.x) s_nodes[k] = nodes[k];
@@ -139,47 +144,34 @@ __global__ void __launch_bounds__(128) k_order_block(float4* __restrict__ nodes,
         }
         __syncthreads();
     }
-    for (int t = threadIdx.x; t < st.treelets; t += blockDim.x) write_treelet(s_nodes, nodes, p, t);
+    for (int t = threadIdx.x; t < st.treelets; t += blockDim.x) write_treelet(s_nodes, ordered, p, t);
     // (Places left over belong to nodes that the root does not reach: both sides unused.)
     const float none = __int_as_float(-1);
-    for (int k = 4 * st.nodes + int(threadIdx.x); k < 4 * n; k += blockDim.x) nodes[k] = make_float4(none, none, none, none);
+    for (int k = 4 * st.nodes + int(threadIdx.x); k < 4 * n; k += blockDim.x) ordered[k] = make_float4(none, none, none, none);
     if (threadIdx.x == 0) *root_size = p.size[0];
 }
 
 }  // namespace
 
-int order_by_treelets(DeviceBuffer<float4>& nodes, int num_nodes, int levels, int* word, cudaStream_t stream) {
-    int size = 0;
-    if (num_nodes <= kBlockTree) {
-        k_order_block<<<1, 128, 0, stream>>>(nodes.ptr, num_nodes, word);
+void order_by_treelets(const float4* nodes, float4* ordered, int* work, int num_nodes, int levels, int* root_size, cudaStream_t stream) {
+    if (num_nodes <= kTreeletBlock) {
+        k_order_block<<<1, 128, 0, stream>>>(nodes, ordered, num_nodes, root_size);
         PTW_CUDA(cudaGetLastError());
-        PTW_CUDA(cudaMemcpyAsync(&size, word, sizeof(int), cudaMemcpyDeviceToHost, stream));
-        PTW_CUDA(cudaStreamSynchronize(stream));
-        return size;
+        return;
     }
     const size_t n = size_t(num_nodes);
-    DeviceBuffer<float4> ordered;
-    DeviceBuffer<int> work;  // the places, then the levels' state
-    if (!ordered.try_allocate(4 * n) || !work.try_allocate(4 * n + sizeof(Levels) / sizeof(int))) return 0;
-    const Places p{work.ptr, work.ptr + n, work.ptr + 2 * n, work.ptr + 3 * n};
-    Levels* st = reinterpret_cast<Levels*>(work.ptr + 4 * n);
-    const Levels first{0, 0, 1, 0};
-    PTW_CUDA(cudaMemcpyAsync(st, &first, sizeof(first), cudaMemcpyHostToDevice, stream));
+    const Places p{work, work + n, work + 2 * n, work + 3 * n};
+    Levels* st = reinterpret_cast<Levels*>(work + 4 * n);
     PTW_CUDA(cudaMemsetAsync(p.size, 0, n * sizeof(int), stream));
-    PTW_CUDA(cudaMemsetAsync(p.root, 0, sizeof(int), stream));
     const int blocks = std::min((num_nodes + 127) / 128, 148 * 16);  // bound by dependent loads: all the warps an SM holds
     for (int level = 0; level < levels; level++) {  // a level of treelets covers at least one of the tree
-        k_next_level<<<1, 1, 0, stream>>>(st);
-        k_choose<<<blocks, 128, 0, stream>>>(nodes.ptr, p, st);
+        k_next_level<<<1, 1, 0, stream>>>(p, st, level == 0);
+        k_choose<<<blocks, 128, 0, stream>>>(nodes, p, st);
     }
     // (Nodes that the root does not reach leave places over: both sides unused.)
-    PTW_CUDA(cudaMemsetAsync(ordered.ptr, 0xff, ordered.bytes(), stream));
-    k_write<<<blocks, 128, 0, stream>>>(nodes.ptr, ordered.ptr, p, st);
+    PTW_CUDA(cudaMemsetAsync(ordered, 0xff, 4 * n * sizeof(float4), stream));
+    k_write<<<blocks, 128, 0, stream>>>(nodes, ordered, p, st, root_size);
     PTW_CUDA(cudaGetLastError());
-    PTW_CUDA(cudaMemcpyAsync(&size, p.size, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    PTW_CUDA(cudaStreamSynchronize(stream));
-    nodes = std::move(ordered);
-    return size;
 }
 
 }  // namespace ptw

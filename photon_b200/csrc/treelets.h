@@ -8,17 +8,19 @@
 namespace ptw {
 
 constexpr int kTreelet = 8;
+constexpr int kTreeletBlock = 512;  // nodes of a tree that one block orders
 
-template <typename T>
-struct DeviceBuffer;
+// The ints of scratch that a tree takes.
+inline size_t treelet_work(int num_nodes) { return 4 * size_t(num_nodes) + 4; }
 
-// Puts the device-resident tree into treelet order (the root stays node 0) and returns the size of the root's
-// treelet, or 0, with the nodes as they were, where there is no memory for the second copy that this takes
-// meanwhile. In the new order the count word of an inner child, which is 0 or less, says more:
+// Writes the tree of `nodes` in treelet order to `ordered` (the root stays node 0) and the size of the root's
+// treelet to *root_size, all on the device, in stream order. Up to kTreeletBlock nodes the two may be one array and
+// `work` null; else they are apart and `work` has treelet_work ints. In the new order the count word of an inner
+// child, which is 0 or less, says more:
 //   -1 .. -8     the child starts another treelet, of that many nodes;
 //   -16 * mask   it belongs to its parent's treelet; the mask has a bit per way out below it, a leaf or another
 //                treelet: bit k for side 0 of the treelet's node k, 8 + k for side 1. Parents precede children.
-// `levels`: bvh_levels of the tree, at least 1. `word`: an int of device scratch. Synchronises the stream.
-int order_by_treelets(DeviceBuffer<float4>& nodes, int num_nodes, int levels, int* word, cudaStream_t stream);
+// `levels`: the tree's (bvh_levels), at least 1.
+void order_by_treelets(const float4* nodes, float4* ordered, int* work, int num_nodes, int levels, int* root_size, cudaStream_t stream);
 
 }  // namespace ptw

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from photon_b200 import abi, native, workloads
+from test_deep_stack import _deep_scene
 from test_gpu_list_walk import _unnested
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +64,16 @@ def test_an_irregular_scene_joins():
     for k in (0, 1, 0):
         assert np.array_equal(image((first, second)[k]), want[k]) and np.array_equal(frame((first, second)[k]), frames[k])
     s.close()
+
+
+def test_the_walks_an_upload_allows():
+    """A built tree is walked out of order, one deeper than the list walk's stack is not, whichever came before."""
+    g = native.terrain_scene(65536, 2)
+    b = g.build()
+    deep, keep = _deep_scene()
+    odd, keep2 = _unnested(b.desc)
+    r = native.Renderer()
+    for desc, walks in ((b.desc, (1, 1)), (deep, (0, 0)), (odd, (0, 0)), (b.desc, (1, 1))):
+        r.upload(desc)
+        assert r.scene_walks() == walks
+    r.close()
