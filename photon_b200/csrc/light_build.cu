@@ -3,8 +3,9 @@
 // materials / lights / environment for a scene already on the device. The definitions, and the order
 // of every floating-point operation, are those of the host builder (scene_build.cpp), so the tables
 // equal the ones pt_scene_build produces for the same inputs; the parallel steps are those whose
-// results do not depend on order (per triangle, per row), the sums that do are taken by one thread
-// in the host's order.
+// results do not depend on order (per triangle, per term, per division), the sums that do are chained by
+// one thread in the host's order (a row's by one of its block), but for the mean luminance, whose rounding
+// is proven from sums in any order (k_env_mean).
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
@@ -149,8 +150,7 @@ __global__ void k_light_alias(const float* __restrict__ w, int n, float4* __rest
     for (; o < no; o++) table[over[o]].x = 1.0f;
 }
 
-// Environment texels with their luminance, and each row's conditional CDF (one thread per row, in
-// the host's order).
+// Environment texels with their luminance.
 __global__ void k_env_texels(const float* __restrict__ rgb, size_t n, float4* __restrict__ out) {
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -243,8 +243,10 @@ __global__ void __launch_bounds__(256) k_env_sums(const float4* __restrict__ tex
 
 // The mean luminance as the host rounds it: the float nearest to (the sum in texel order) / n. Any two
 // orders of n double additions differ by at most 2 n u sum |l| (u = 2^-53), so when both ends of that
-// interval round to one float, it is the host's; otherwise (about one image in 500) one thread takes the
-// sum in order. That chain, which was the whole of it, is 13 ms for a 1024x512 image.
+// interval round to one float, it is the host's; otherwise one thread takes the sum in order. That chain,
+// which was the whole of it, is 13 ms for a 1024x512 image and grows with n. So does how often it is taken: the
+// interval is 4.2 n u wide, a float's spacing 2^-24 to 2^-23, so about one image in 250 to 500 of 1024x512 and one in
+// 4 to 8 of 8192x4096, where it takes the better part of a second.
 __global__ void k_env_mean(const float4* __restrict__ texels, size_t n, const double* __restrict__ sums, float* __restrict__ scalars) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const double slack = 2.1 * double(n) * 0x1p-53 * sums[1];
