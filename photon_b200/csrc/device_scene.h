@@ -49,13 +49,9 @@ struct DeviceBuffer {
         count = 0;
     }
     void allocate(size_t n) {
-        if (n == count && ptr) return;
-        release();
-        if (n == 0) return;
-        PTW_CUDA(cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T)));
-        count = n;
+        if (!try_allocate(n)) throw Error{PT_ERR_CUDA, "CUDA error: out of memory (cudaMalloc)"};
     }
-    // allocate() for what can be done without: false, with nothing held, where there is no memory for it.
+    // False, with nothing held and no error left behind for a later call to find, where there is no memory.
     bool try_allocate(size_t n) {
         if (n == count && ptr) return true;
         release();

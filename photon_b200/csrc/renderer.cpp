@@ -97,6 +97,7 @@ void WavefrontEngine::reserve_paths(uint64_t needed) {
     uint64_t want = std::min<uint64_t>(uint64_t(tuning_.path_capacity), (needed + 1023) / 1024 * 1024);
     if (want < 1024) want = 1024;
     if (pb_.capacity >= want) return;
+    pb_ = PathBuffers{};  // (nothing of the old pool is valid if an allocation below fails)
     for (auto& b : bufs_) b.allocate(want);
     for (auto& b : ids_) b.allocate(want);
     for (int k = 0; k < 2; k++) {

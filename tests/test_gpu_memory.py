@@ -58,6 +58,34 @@ def test_a_light_rebuild_keeps_little(cuda):
     assert held <= (32 << 20) + SLACK
 
 
+def test_a_pool_that_cannot_grow_leaves_the_renderer_usable(cuda):
+    import torch
+    g = native.terrain_scene(65536, 2)
+    b = g.build()
+    cam = g.camera(16 / 9)
+    r = native.Renderer()
+    r.upload(b.desc)
+
+    def image(w, h, spp):
+        r.resize(w, h)
+        r.reset()
+        r.render(cam, abi.render_settings(w, h, max_depth=4, seed=2), spp)
+        return r.download_accumulation()
+
+    want = image(160, 90, 4)
+    r.resize(1280, 720)
+    held = torch.empty(max(0, _free(cuda) - (700 << 20)), dtype=torch.uint8, device="cuda")  # room for the samples, not for the paths
+    try:
+        with pytest.raises(native.PhotonError):
+            r.render(cam, abi.render_settings(1280, 720, max_depth=4, seed=2), 16)
+        again = image(160, 90, 4)
+    finally:
+        held = None
+        torch.cuda.empty_cache()
+        r.close()
+    assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("kind", ["box", "terrain"])
 def test_the_class_order_beside_sorted_shadow_rays(kind):
     """The order of the shading and that of the shadow walk share their memory: an iteration that has both."""
