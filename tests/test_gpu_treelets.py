@@ -64,3 +64,22 @@ def test_nodes_that_the_root_does_not_reach(n):
     d = abi.SceneDesc.from_buffer_copy(b.desc)
     d.nodes = nodes
     _check(d, (1, 1))
+
+
+def test_new_lights_keep_the_order():
+    b = _patch(3000)
+    w, h = 96, 64
+    center, extent = workloads.scene_sphere(b.desc)
+    cam = workloads.look_at(np.asarray(center) + 0.8 * extent * np.array([0.3, 1.0, 0.2]), center, 60.0, w / h)
+    out = []
+    for again in (False, True):
+        r = native.Renderer()
+        r.upload(b.desc)
+        if again:
+            r.update_lights(b.desc)
+        assert r.scene_walks() == (1, 1)
+        r.resize(w, h)
+        r.render(cam, abi.render_settings(w, h, max_depth=6, seed=3), 2)
+        out.append(r.download_accumulation())
+        r.close()
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
