@@ -252,7 +252,7 @@ typedef struct pt_tuning {
                                   thread per path); 0 never; -1 keep; -2 (default) 16,384 for a render that
                                   starts while no other render of this process runs on the device, 8,192
                                   beside one or two others, on a scene of fewer than 1,024 BVH nodes and in
-                                  the server, 4,096 beside more; on trees that cannot be walked out of
+                                  the server, 1,024 beside more; on trees that cannot be walked out of
                                   order (the stack or the boxes are irregular) 131,072 and 65,536 */
     int32_t wide_shadows;      /* 1: shadow rays walk a 4-wide BVH collapsed from the scene's BVH2 (same
                                   answers), 0 (default): the BVH2; -1 keep */

@@ -25,15 +25,15 @@ constexpr int kTailAlone = 1 << 17;
 constexpr int kTailShared = 1 << 16;
 // The same where the tail walks rays by groups of eight lanes (WfParams::group_tail): it takes half the time
 // of a thread per path up to 16,384 paths and loses above, and beside other renders it yields sooner.
-// Terrain of 262K triangles, 57,600 paths alone: 1.12 ms with 131,072, 0.93 with 16,384; 1600x900 real-time
-// frames, frames/s with 131,072 (alone) or 65,536 / 16,384 / 8,192 / 4,096: one session 399 / 436 / 401 /
-// 376, two 599 / 600 / 598 / 580, four 699 / 703 / 766 / 770, eight 706 / 704 / 803 / 851.
+// 1600x900 real-time frames of the 262K terrain, frames/s with 131,072 / 65,536 / 16,384 / 8,192 / 4,096: one
+// session 410 / 435 / 435 / 415 / 400, two 533 / 589 / 590 / 607 / 601; with 8,192 / 4,096 / 2,048 / 1,024 / 512:
+// four 729 / 745 / 769 / 773 / 755, eight 742 / 785 / 806 / 827 / 829.
 constexpr int kGroupTailAlone = 1 << 14;
 constexpr int kGroupTailFew = 1 << 13;   // one or two other renders; or a tree of fewer than kSmallTree nodes
 // Frames of 16,384 paths, ms with 16,384 / 8,192, over trees of 19 nodes: 0.33 / 0.29, 138: 0.33 / 0.26,
 // 268: 0.38 / 0.30, 541: 0.41 / 0.35; 1,072: 0.28 / 0.30, 2,150: 0.35 / 0.37, 16,859: 0.56 / 0.57.
 constexpr int kSmallTree = 1024;
-constexpr int kGroupTailMany = 1 << 12;
+constexpr int kGroupTailMany = 1 << 10;  // three or more others
 
 // Tunable launch parameters (the autotuner's knobs).
 struct Tuning {
