@@ -487,7 +487,8 @@ def main():
                                   "960x540x4 profile case, times this frame's rays per launch",
                 "algorithmic_bytes_per_launch": trace_bytes_per_frame * args.steps / trace_launches,
                 "avg_launch_ms": prof.trace.ms / trace_launches,
-                "model": "64 B per node visit + 48 B per triangle test (closest-hit rays)",
+                "model": "64 B per node visit + 48 B per triangle test of Photon's walk (closest-hit rays), counted by the pair walk, "
+                         "which makes exactly those; the timed list walk visits about 4% more nodes",
                 "node_visits_per_ray": counts.closest_node_visits / max(1, counts.closest_rays),
                 "tri_tests_per_ray": counts.closest_tri_tests / max(1, counts.closest_rays),
                 # SIMT use of the two walks: from the counted render, the lanes that visit a node per
