@@ -160,6 +160,7 @@ void DeviceScene::upload(const pt_scene_desc& d, cudaStream_t s, bool lights_onl
     if (lights_only && !ready_) lights_only = false;
     if (lights_only && d.num_tris != view_.num_tris) throw Error{PT_ERR_INVALID, "update_lights: the triangle count changed"};
     const int levels = validate_scene(d, lights_only);
+    ready_ = false;  // (until the last array is there: a failure below leaves parts of two scenes)
     if (!lights_only) {
         d_view_.allocate(1);
         light_work_.release();

@@ -86,6 +86,35 @@ def test_a_pool_that_cannot_grow_leaves_the_renderer_usable(cuda):
     assert np.array_equal(again.view(np.uint32), want.view(np.uint32))
 
 
+def test_an_upload_that_fails_leaves_no_scene(cuda):
+    import torch
+    small, big = native.terrain_scene(65536, 2), native.terrain_scene(1 << 21, 2)
+    b, c = small.build(), big.build(gpu=True)
+    cam, rs = small.camera(16 / 9), abi.render_settings(160, 90, max_depth=4, seed=2)
+    r = native.Renderer()
+    r.resize(160, 90)
+    images = []
+    for again in (False, True):
+        r.upload(b.desc)
+        r.reset()
+        r.render(cam, rs, 2)
+        images.append(r.download_accumulation())
+        if again:
+            break
+        held = torch.empty(max(0, _free(cuda) - (120 << 20)), dtype=torch.uint8, device="cuda")  # the big scene takes 350 MB
+        try:
+            with pytest.raises(native.PhotonError):
+                r.upload(c.desc)
+            with pytest.raises(native.PhotonError) as e:
+                r.render(cam, rs, 2)
+        finally:
+            held = None
+            torch.cuda.empty_cache()
+        assert e.value.code == abi.PT_ERR_NO_SCENE
+    r.close()
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+
+
 @pytest.mark.parametrize("kind", ["box", "terrain"])
 def test_the_class_order_beside_sorted_shadow_rays(kind):
     """The order of the shading and that of the shadow walk share their memory: an iteration that has both."""
